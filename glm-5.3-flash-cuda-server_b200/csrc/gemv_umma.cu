@@ -43,8 +43,9 @@
 // in the shared memory of the next CTA on that SM.
 // Prologue without a CTA-wide barrier: warp 0 initialises the barriers of its own loads and requests the
 // slabs and the first four stages at once; the MMA warps initialise the other barriers, allocate TMEM and
-// arrive at named barrier 3, where only the producer waits; the workers go straight to the dependency
-// wait and the activation loads, and learn of everything else at named barrier 2.
+// arrive at named barrier 3, where only the producer waits, and wait at named barrier 4, where the producer
+// arrives once its barriers are initialised; the workers go straight to the dependency wait and the
+// activation loads, and learn of everything else at named barrier 2.
 //
 // Decode kernel with RESIDENT scales (RES: up to four activation rows, one tile per CTA, K <= 7424 for one
 // row, 6912 for two, 5888 for three or four): TMEM has room for the scales of every step at once, so the MMA
@@ -329,6 +330,7 @@ k_gemv_umma(const __grid_constant__ UmParams p, const __grid_constant__ UmMaps m
         if (lane == 0) mbar_init(smem_u32(&sc_bar), 1);
         mbar_fence_init();
         __syncwarp();
+        asm volatile("bar.arrive 4, %0;" :: "r"(32 + 32 * UM_MMA_WARPS) : "memory");      // the MMA warps wait on these barriers before anyone else does
         if (early_scales) {
             issue_scales();
             for (int g = lane; g < n_early; g += 32) issue_stage(g);
@@ -353,12 +355,14 @@ k_gemv_umma(const __grid_constant__ UmParams p, const __grid_constant__ UmMaps m
         }
         tc_fence_before();
     }
-    // The producer waits at barrier 3 for the MMA warps' initialisations; they only arrive there (the
-    // producer has nothing they need) and meet among themselves at barrier 4 for the TMEM address.
+    // The producer waits at barrier 3 for the MMA warps' initialisations; they only arrive there.  They meet at
+    // barrier 4 for the TMEM address and for the producer's initialisations: they wait on sc_bar and full_bar
+    // before the CTA's other barriers, and a wait on a word that the previous CTA of the SM left there, its
+    // phase complete, would let them read scales that have not landed.
     if (warp == 0) named_sync(3, 32 + 32 * UM_MMA_WARPS);
     if (mma_warp) {
         asm volatile("bar.arrive 3, %0;" :: "r"(32 + 32 * UM_MMA_WARPS) : "memory");
-        named_sync(4, 32 * UM_MMA_WARPS);
+        named_sync(4, 32 + 32 * UM_MMA_WARPS);
     }
     uint32_t tmem = 0u, tq = 0u;                     // TMEM base; the lane quadrant this warp may access (set once the role knows the base)
     // Weight scales, shared memory -> TMEM.  Lane l holds rows l, l+32, l+64, l+96: 16 bytes each = four
