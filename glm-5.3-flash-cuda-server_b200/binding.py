@@ -141,8 +141,17 @@ def stream_ptr(stream=None):
     return C.c_void_p(s.cuda_stream)
 
 
+def _stream(stream):
+    """The cudaStream_t as an int (an argument of type c_void_p takes one without an object in between).
+    torch.cuda.current_stream() builds a Stream object (3.4 us, as long as a whole launch); the raw handle of the
+    same stream takes 0.1 us."""
+    if stream is not None:
+        return stream.cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def _ptr(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else C.c_void_p(0)
+    return t.data_ptr() if t is not None else None
 
 
 class Nvfp4Weight:
@@ -185,9 +194,9 @@ def gemm(W, x, y=None, dtype=BF16, stream=None, ws=None):
     if y is None:
         y = torch.empty((M, N), dtype=torch.float32, device=x.device)
     if ws is not None:
-        check(lib().b200_nvfp4_gemm_ws(_ptr(y), C.byref(ref), _ptr(x2), M, N, K, dtype, _ptr(ws), stream_ptr(stream)), 'b200_nvfp4_gemm_ws')
+        check(lib().b200_nvfp4_gemm_ws(_ptr(y), C.byref(ref), _ptr(x2), M, N, K, dtype, _ptr(ws), _stream(stream)), 'b200_nvfp4_gemm_ws')
     else:
-        check(lib().b200_nvfp4_gemm(_ptr(y), C.byref(ref), _ptr(x2), M, N, K, dtype, stream_ptr(stream)), 'b200_nvfp4_gemm')
+        check(lib().b200_nvfp4_gemm(_ptr(y), C.byref(ref), _ptr(x2), M, N, K, dtype, _stream(stream)), 'b200_nvfp4_gemm')
     return y if x.dim() == 2 else y[0]
 
 
@@ -204,7 +213,7 @@ def gemm_bf16(W, x_bf16, y=None, ws=None, stream=None):
     if ws is None:
         ws = gemm_bf16_workspace(M, K, x_bf16.device)
     ref = W.wref()
-    check(lib().b200_nvfp4_gemm_bf16(_ptr(y), C.byref(ref), _ptr(x_bf16), M, W.N, K, _ptr(ws), stream_ptr(stream)), 'b200_nvfp4_gemm_bf16')
+    check(lib().b200_nvfp4_gemm_bf16(_ptr(y), C.byref(ref), _ptr(x_bf16), M, W.N, K, _ptr(ws), _stream(stream)), 'b200_nvfp4_gemm_bf16')
     return y
 
 
@@ -217,7 +226,7 @@ def gemm_bf16_exact(W, x_bf16, y=None, ws=None, stream=None):
     if ws is None:
         ws = torch.empty(lib().b200_nvfp4_gemm_bf16_exact_workspace_bytes(M, K), dtype=torch.uint8, device=x_bf16.device)
     ref = W.wref()
-    check(lib().b200_nvfp4_gemm_bf16_exact(_ptr(y), C.byref(ref), _ptr(x_bf16), M, W.N, K, _ptr(ws), stream_ptr(stream)), 'b200_nvfp4_gemm_bf16_exact')
+    check(lib().b200_nvfp4_gemm_bf16_exact(_ptr(y), C.byref(ref), _ptr(x_bf16), M, W.N, K, _ptr(ws), _stream(stream)), 'b200_nvfp4_gemm_bf16_exact')
     return y
 
 
@@ -230,7 +239,7 @@ def quantize_tokens(x, stream=None):
     sfb = torch.empty((K // 256, M, 16), dtype=torch.uint8, device=dev)
     gs = torch.empty(M, dtype=torch.float32, device=dev)
     check(lib().b200_nvfp4_quantize_tokens(_ptr(x), 1 if x.dtype == torch.float32 else 0, M, K, _ptr(packed), _ptr(sfb), _ptr(gs),
-                                           stream_ptr(stream)), 'b200_nvfp4_quantize_tokens')
+                                           _stream(stream)), 'b200_nvfp4_quantize_tokens')
     return packed, sfb.permute(1, 0, 2).reshape(M, K // 16).contiguous(), gs
 
 
@@ -247,7 +256,7 @@ def dense_mlp(x, gate, up, down, limit=10.0, y=None, ws=None, stream=None):
     if ws is None:
         ws = dense_mlp_workspace(M, H, I, x.device)
     g, u, d = gate.wref(), up.wref(), down.wref()
-    check(lib().b200_dense_mlp(_ptr(x), C.byref(g), C.byref(u), C.byref(d), H, I, float(limit), _ptr(y), _ptr(ws), M, stream_ptr(stream)),
+    check(lib().b200_dense_mlp(_ptr(x), C.byref(g), C.byref(u), C.byref(d), H, I, float(limit), _ptr(y), _ptr(ws), M, _stream(stream)),
           'b200_dense_mlp')
     return y
 
@@ -272,21 +281,21 @@ def gemv_multi(weights, xs, M=1, ys=None, stream=None, jobs=None, ws=None):
     if jobs is None:
         jobs = make_jobs(weights, xs, ys)
     if ws is not None:
-        check(lib().b200_nvfp4_gemv_multi_ws(jobs, len(weights), M, weights[0].K, BF16, _ptr(ws), stream_ptr(stream)), 'b200_nvfp4_gemv_multi_ws')
+        check(lib().b200_nvfp4_gemv_multi_ws(jobs, len(weights), M, weights[0].K, BF16, _ptr(ws), _stream(stream)), 'b200_nvfp4_gemv_multi_ws')
     else:
-        check(lib().b200_nvfp4_gemv_multi(jobs, len(weights), M, weights[0].K, BF16, stream_ptr(stream)), 'b200_nvfp4_gemv_multi')
+        check(lib().b200_nvfp4_gemv_multi(jobs, len(weights), M, weights[0].K, BF16, _stream(stream)), 'b200_nvfp4_gemv_multi')
     return ys
 
 
 def f32_to_bf16(src, stream=None):
     dst = torch.empty(src.shape, dtype=torch.bfloat16, device=src.device)
-    check(lib().b200_f32_to_bf16(_ptr(dst), _ptr(src), src.numel(), stream_ptr(stream)), 'b200_f32_to_bf16')
+    check(lib().b200_f32_to_bf16(_ptr(dst), _ptr(src), src.numel(), _stream(stream)), 'b200_f32_to_bf16')
     return dst
 
 
 def bf16_to_f32(src, stream=None):
     dst = torch.empty(src.shape, dtype=torch.float32, device=src.device)
-    check(lib().b200_bf16_to_f32(_ptr(dst), _ptr(src), src.numel(), stream_ptr(stream)), 'b200_bf16_to_f32')
+    check(lib().b200_bf16_to_f32(_ptr(dst), _ptr(src), src.numel(), _stream(stream)), 'b200_bf16_to_f32')
     return dst
 
 
@@ -299,14 +308,14 @@ def quantize(w_bf16, gscale_in=None, out=None, stream=None):
                           torch.empty((N, K // 16), dtype=torch.uint8, device=dev),
                           torch.empty(1, dtype=torch.float32, device=dev), device=dev)
     check(lib().b200_nvfp4_quantize(_ptr(w_bf16), N, K, _ptr(out.packed), _ptr(out.scale), _ptr(out.gscale),
-                                    _ptr(gscale_in), stream_ptr(stream)), 'b200_nvfp4_quantize')
+                                    _ptr(gscale_in), _stream(stream)), 'b200_nvfp4_quantize')
     return out
 
 
 def dequantize(W, stream=None):
     out = torch.empty((W.N, W.K), dtype=torch.float32, device=W.packed.device)
     m = W.mat()
-    check(lib().b200_nvfp4_dequantize(_ptr(out), C.byref(m), W.N, W.K, stream_ptr(stream)), 'b200_nvfp4_dequantize')
+    check(lib().b200_nvfp4_dequantize(_ptr(out), C.byref(m), W.N, W.K, _stream(stream)), 'b200_nvfp4_dequantize')
     return out
 
 
@@ -348,7 +357,7 @@ def moe_route(layer, x, stream=None):
     sel = torch.empty((M, layer.topk), dtype=torch.int32, device=x.device)
     wts = torch.empty((M, layer.topk), dtype=torch.float32, device=x.device)
     logits = torch.empty((M, layer.n_expert), dtype=torch.float32, device=x.device)
-    check(lib().b200_moe_route(_ptr(x2), C.byref(layer.c), _ptr(sel), _ptr(wts), _ptr(logits), M, stream_ptr(stream)), 'b200_moe_route')
+    check(lib().b200_moe_route(_ptr(x2), C.byref(layer.c), _ptr(sel), _ptr(wts), _ptr(logits), M, _stream(stream)), 'b200_moe_route')
     return sel, wts, logits
 
 
@@ -360,7 +369,7 @@ def moe_forward(layer, x, y=None, sel=None, wts=None, stream=None):
     sel = torch.empty((M, layer.topk), dtype=torch.int32, device=dev) if sel is None else sel
     wts = torch.empty((M, layer.topk), dtype=torch.float32, device=dev) if wts is None else wts
     ws = layer.workspace(M)
-    check(lib().b200_moe_forward(_ptr(x2), C.byref(layer.c), _ptr(y), _ptr(sel), _ptr(wts), _ptr(ws), M, stream_ptr(stream)), 'b200_moe_forward')
+    check(lib().b200_moe_forward(_ptr(x2), C.byref(layer.c), _ptr(y), _ptr(sel), _ptr(wts), _ptr(ws), M, _stream(stream)), 'b200_moe_forward')
     return y, sel, wts
 
 
@@ -383,7 +392,7 @@ def moe_experts(layer, x, sel, wts, y=None, stream=None):
     M = x2.shape[0]
     y = torch.empty((M, layer.hidden), dtype=torch.float32, device=x.device) if y is None else y
     ws = layer.workspace(M)
-    check(lib().b200_moe_experts(_ptr(x2), C.byref(layer.c), _ptr(y), _ptr(sel), _ptr(wts), _ptr(ws), M, stream_ptr(stream)), 'b200_moe_experts')
+    check(lib().b200_moe_experts(_ptr(x2), C.byref(layer.c), _ptr(y), _ptr(sel), _ptr(wts), _ptr(ws), M, _stream(stream)), 'b200_moe_experts')
     return y
 
 
@@ -395,7 +404,7 @@ def moe_forward_static(layer, x, y=None, sel=None, wts=None, stream=None):
     y = torch.empty((M, layer.hidden), dtype=torch.float32, device=dev) if y is None else y
     sel = torch.empty((M, layer.topk), dtype=torch.int32, device=dev) if sel is None else sel
     wts = torch.empty((M, layer.topk), dtype=torch.float32, device=dev) if wts is None else wts
-    check(lib().b200_moe_forward_static(_ptr(x2), C.byref(layer.c), _ptr(y), _ptr(sel), _ptr(wts), M, stream_ptr(stream)),
+    check(lib().b200_moe_forward_static(_ptr(x2), C.byref(layer.c), _ptr(y), _ptr(sel), _ptr(wts), M, _stream(stream)),
           'b200_moe_forward_static')
     return y, sel, wts
 
@@ -422,7 +431,7 @@ class EpContext:
         y = torch.empty((T, self.router.hidden), dtype=torch.float32, device=dev) if y is None else y
         sel = torch.empty((T, self.router.topk), dtype=torch.int32, device=dev) if sel is None else sel
         wts = torch.empty((T, self.router.topk), dtype=torch.float32, device=dev) if wts is None else wts
-        check(lib().b200_ep_forward(self.h, _ptr(x), _ptr(y), _ptr(sel), _ptr(wts), T, stream_ptr(stream)), 'b200_ep_forward')
+        check(lib().b200_ep_forward(self.h, _ptr(x), _ptr(y), _ptr(sel), _ptr(wts), T, _stream(stream)), 'b200_ep_forward')
         return y, sel, wts
 
     def stats(self):
