@@ -85,16 +85,26 @@ int umma_table_launch(const UmJob* table, int n_jobs, int N, int K, int R, float
 
 // gemm_mxf4.cu: the wide GEMM with both operands in NVFP4 (activations quantised per token first).
 // One job: `rows` activation rows, starting at row `row0` of the quantised activation buffer, against one
-// weight matrix of N rows; y[m * ldy + n].  gs_x points at the job's first per-token global scale.
-// mw, ms: tensor maps of the weight in GLOBAL memory (table launches; box height = the launch's R).
-struct GxJob { float* y; const float* gs_w; const float* gs_x; const void* mw; const void* ms; int row0; int rows; int N; int ldy; };
+// weight matrix of N rows; y[m * ldy + n].  gs_x points at the job's first per-token global scale, sfb at its
+// block of activation scales (layout: ActQuant).  mw: tensor map of the packed weights in GLOBAL memory (table
+// launches; box height 128), sc: their scale bytes.  mw2, sc2, gs_w2: the second matrix of a dual launch (gate and
+// up of an expert), whose output is the clamped SwiGLU of the two products.
+struct GxJob { float* y; const float* gs_w; const float* gs_w2; const float* gs_x; const void* mw; const void* mw2;
+               const unsigned char* sc; const unsigned char* sc2; const unsigned char* sfb; int row0; int rows; int N; int ldy; };
 size_t gemm_mxf4_ws_bytes(int M, int K);
 bool gemm_mxf4_shape_ok(int K);
 int gemm_mxf4_dense(float* y, const b200_wref* W, const void* x, int x_kind, int M, int N, int K, void* ws, cudaStream_t s);
-int quant_act_launch(int mode, const void* x, const void* x2, float limit, const int* src_row, const int* m_dev, int M,
-                     int rows_launch, int K, unsigned char* xq, unsigned char* sfb, size_t sfb_rows, float* gsx, cudaStream_t s);
-int gemm_mxf4_table(const GxJob* table, int max_jobs, long expected_jobs, int NT, int N, int K, int R, const unsigned char* xq, size_t x_rows,
-                    const unsigned char* sfb, size_t sfb_rows, cudaStream_t s);
+// Where the activation quantiser puts a row.  sfb is a sequence of blocks, one per job (a job's NT token columns padded to
+// nblk * 128), each [K/256 steps][nblk][four 64-k blocks][32][16 B]: token c*32 + l of a 128-token block has its four scale
+// bytes of a 64-k block at [l][4c..4c+3], which is what tcgen05.cp 32x128b moves to the TMEM columns the MMA reads.
+// Source row r goes to ndst destinations: packed row pos[r * ndst + d] (pos == nullptr: row r) and scale slot
+// sfrow[r * ndst + d] = job * nblk * 128 + column (sfrow == nullptr: token r, jobs of NT tokens).
+struct ActQuant { unsigned char* xq; unsigned char* sfb; float* gsx; const int* pos; const int* sfrow; int ndst; int NT; int nblk; };
+int quant_act_launch(int x_is_f32, const void* x, int M, int K, const ActQuant& q, cudaStream_t s);
+// Jobs from a table in device memory, *n_jobs of them; dual: gate and up at once, SwiGLU written.
+int gemm_mxf4_table(const GxJob* table, const int* n_jobs, int NT, int N, int K, bool dual, float limit, const unsigned char* xq,
+                    size_t x_rows, cudaStream_t s);
+__host__ __device__ inline int gx_blocks(int NT) { return (NT + 127) / 128; }
 
 // gemm_f16w.cu: the exact wide GEMM (weights dequantised to fp16 in the kernel, tcgen05 kind::f16).
 size_t gemm_f16w_ws_bytes(int M, int K);

@@ -1,62 +1,55 @@
 // gemm_mxf4.cu -- the wide (prefill / batched, M >= 16) NVFP4 GEMM: y[M,N] = x[M,K] . W[N,K]^T on
 // tcgen05.mma kind::mxf4nvf4.block_scale.block16 with BOTH operands in NVFP4.
 //
-// The weights are used exactly as the format stores them (packed e2m1 bytes and e4m3 block
-// scales, read through TMA).  The activations are quantised to NVFP4 first, one token at a time,
-// by k_quant_act: the reference's own quant_block rule (tools/requant_dense_nvfp4.py:53-68) with a
-// per-token global scale 2688 / amax(token), so that a token's result never depends on the rest of
-// its batch.  That costs about 9 % per-element activation error; results are therefore judged against
-// deq(W) . deq(quant(x)), and the library keeps the exact small-batch kernels (gemv_umma.cu) for
-// callers that want fp32-activation accuracy.  The reference streams W once per chunk of 4 rows
-// (kernels/gemv.cu:369-396); here W is read ONCE for up to 256 rows.
+// The weights are used exactly as the format stores them (packed e2m1 bytes and e4m3 block scales).  The
+// activations are quantised to NVFP4 first, one token at a time, by k_quant_act: the reference's own quant_block
+// rule (tools/requant_dense_nvfp4.py:53-68) with a per-token global scale 2688 / amax(token), so that a token's
+// result never depends on the rest of its batch.  That costs about 9 % per-element activation error; results are
+// therefore judged against deq(W) . deq(quant(x)), and the library keeps the exact small-batch kernels
+// (gemv_umma.cu) for callers that want fp32-activation accuracy.  The reference streams W once per chunk of 4 rows
+// (kernels/gemv.cu:369-396); here W crosses HBM once per call.
 //
-// One CTA per (tile of R <= 128 weight rows, job of up to NT activation rows); K walked in steps of
-// 256.  The accumulator D[128 weight rows (lanes), NT tokens (columns)] stays in TMEM for the whole K.
-//   warp 0      TMA producer: the tile's weight scale rows once (slabs [R x 128 B]); per step one
-//               128B-swizzled box of packed weights [128 B x R], one of packed activations
-//               [128 B x NT] and the step's activation scales (one contiguous NT x 16 B chunk: the
-//               quantiser writes them step-major) into a ring of stages.  Lane l issues steps l, l+32, ..
-//   warp 1      MMA issuer: four tcgen05.mma (K = 64 each, N = NT) per step, tcgen05.commit frees the stage
+// Persistent: one CTA per SM walks work items (TA tiles of R <= 128 weight rows) x (a job's NT tokens), K in steps of
+// 256.  The accumulators D[128 weight rows (lanes), NT tokens (columns)] of the TA tiles stay in TMEM for the whole K.
+// What bounds it is the SM's intake from L2, about 64 B per clock: a step of a 128 x NT tile brings 16 KB of weights and
+// NT x 128 B of activations for NT/2 clocks of MMA.  Hence TA = 2: two weight tiles against one activation tile
+// (for a MoE expert its gate and its up tile, so that the SwiGLU is applied where both sums lie and one value instead
+// of two is written).
+//   warp 0      TMA: per step TA 128B-swizzled boxes of packed weights [128 B x R]
+//   warp 3      TMA: per step one box of packed activations [128 B x NT] and their scale bytes (one bulk copy: the
+//               quantiser writes them in the order tcgen05.cp wants)
+//   warps 4-7   weight scales: 16 bytes of 128 rows per step, read straight from global memory one unit (two steps of
+//               a tile) ahead, transposed in registers to [64-k block][32][16 B] in shared memory.  The slabs in
+//               shared memory and the eight warps of tcgen05.st that this replaces held the kernel to three stages
+//   warp 1      MMA issuer: per step tcgen05.cp of both operands' scales to a slot of TMEM columns, then TA x four
+//               tcgen05.mma (K = 64 each); tcgen05.commit frees the stage
 //   warp 2      allocates / frees TMEM
-//   warps 4-11  two groups of four warps (one per TMEM lane quadrant) on alternate steps move the
-//               step's scales into TMEM with tcgen05.st (lane r % 32, column r / 32: the layout the
-//               block-scaled MMA reads): 16 columns for the weights' 128 x 16 scale bytes, NT/8 for the
-//               activations'.  Afterwards each group reads half of the accumulator columns, applies
-//               1 / (gs_w * gs_x[token]) and writes y (lanes = consecutive n: coalesced).
-// Barriers full/sf/empty are per step and used once (K <= 16384: at most 64 steps).  Every wait is
-// bounded (tma_pipe.cuh).  No cluster launch, no multicast.
+//   warps 8-15  epilogue: 1 / (gs_w * gs_x[token]) and the store (lanes = consecutive n: coalesced); with room for
+//               two sets of accumulators it overlaps the next item's MMAs, otherwise the next item's loads
+// Every wait is bounded (tma_pipe.cuh).  No cluster launch, no multicast.
 #include "b200_internal.h"
 #include "quant_core.cuh"
 #include "tma_pipe.cuh"
 #include <cuda.h>
-#include <cstdio>
-#include <cstdlib>
 
 namespace b200 {
 
-constexpr int GX_THREADS = 384;
-constexpr int GX_MOVERS = 256;
-constexpr int GX_MAX_STEPS = 64;                   // K <= 16384
-constexpr int GX_MAX_STAGES = 8;
-constexpr int GX_MAX_SLABS = 16;                   // scale slabs per CTA (a slab covers 8 steps, or a whole tile when K/16 < 128)
-constexpr int GX_TMEM_COLS = 512;                  // accumulator [0, NT) | scale slots from column 256
-constexpr int GX_COL_SF = 256;
-constexpr uint32_t GX_A_BYTES = 16384;             // the MMA always reads 128 rows x 128 B of a stage
+constexpr int GX_THREADS = 512;
+constexpr int GX_MAX_STAGES = 16;
+constexpr int GX_TMEM_COLS = 512;                  // accumulators [0, nbuf * TA * NT) | scale slots
+constexpr int GX_MAX_NT = 256;
 
 struct GxParams {
     const GxJob* table;                            // jobs in global memory (written by an earlier kernel), or nullptr:
-    GxJob one;                                     // ... job j = activation rows [j * NT, j * NT + NT) of `one`
-    const unsigned char* sfb;                      // activation scales [K/256][sfb_rows][16]
-    size_t sfb_rows;
+    const int* n_jobs_dev;                         // ... and how many there are
+    GxJob one;                                     // dense: job j = activation rows [j * NT, j * NT + NT) of `one`
     unsigned int* status;
-    int n_jobs, K, R, prefetch_before_wait;
-    int sa, sb, ssf;                               // slots of the weight ring, of the activation ring, and of the scale slots in TMEM (ssf <= sb)
-    uint32_t a_slot;                               // bytes of a weight slot: R x 128 rounded up to 1 KB (the MMA reads 16 KB from its start)
-    int sc_box, sc_swz;
-    int T;                                         // consecutive weight-row tiles per CTA (T * NT <= 256 accumulator columns, T * K/256 <= 64 steps)
-    int sps, nslot;                                // steps per scale slab; slots of the slab ring
-    int nacc;                                      // accumulators per tile (1, 2 or 4): k-block it adds into accumulator it % nacc
+    int n_jobs, K, R, NT, tiles;                   // tiles: work items per job
+    int stages, nbuf, nslot, nblk, prefetch_before_wait;
+    uint32_t a_slot, b_off, ts_off, sf_off;        // bytes of a weight slot; offsets of the other rings from the first
+    float limit;
 };
+struct GxMaps { CUtensorMap w; CUtensorMap x[4]; };       // dense: weights; activations with boxes of NT rows (table: NT, 64, 32 and 16)
 
 __device__ __forceinline__ void gx_tma_2d(uint32_t dst, const void* map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -66,277 +59,319 @@ __device__ __forceinline__ uint64_t gx_desc(uint32_t saddr) {
     // K-major operand tile, 128B-swizzled: start address >> 4 | SBO = 1024 B (8 rows) | version 1 | SWIZZLE_128B
     return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)(1024u >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
+__device__ __forceinline__ uint64_t gx_desc_sf(uint32_t saddr) {
+    // 32 rows x 16 B of scales, contiguous: four 8-row core matrices 128 B apart, no swizzle
+    return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | ((uint64_t)1 << 46);
+}
 __device__ __forceinline__ void gx_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void gx_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void gx_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
 }
+__device__ __forceinline__ void gx_cp_sf(uint32_t col, uint64_t desc) {
+    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" :: "r"(col), "l"(desc) : "memory");
+}
+__device__ __forceinline__ void gx_ld16(uint32_t col, float (&d)[16]) {
+    uint32_t v[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                 : "r"(col));
+    #pragma unroll
+    for (int j = 0; j < 16; ++j) d[j] = __uint_as_float(v[j]);
+}
+// The item's job and its weight-row tile.  A table's items go job by job (the tiles of an expert run side by side and
+// share its activation tile in L2), a dense call's tile by tile (the token chunks of a weight tile share the weights).
+struct GxItem { int job, tile; };
+template <bool TABLE>
+__device__ __forceinline__ GxItem gx_item(const GxParams& p, int idx) {
+    GxItem q;
+    if (TABLE) { q.job = idx / p.tiles; q.tile = idx - q.job * p.tiles; }
+    else { q.tile = idx / p.n_jobs; q.job = idx - q.tile * p.n_jobs; }
+    return q;
+}
+template <bool TABLE>
+__device__ __forceinline__ GxJob gx_job(const GxParams& p, int job) {
+    if (TABLE) return p.table[job];
+    GxJob J = p.one;
+    J.row0 = job * p.NT;
+    J.rows = min(p.NT, J.rows - J.row0);
+    J.y += (size_t)J.row0 * J.ldy;
+    J.gs_x += J.row0;
+    J.sfb += (size_t)job * (p.K >> 8) * p.nblk * 2048;
+    return J;
+}
 
-// tcgen05.st of 4*CB registers (32x32b): register i goes to column i of the warp's lane quadrant.
-template <int N> struct GxSt;
-template <> struct GxSt<4> {
-    static __device__ __forceinline__ void st(uint32_t a, const uint32_t* r) {
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};"
-                     :: "r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
-    }
-};
-template <> struct GxSt<8> {
-    static __device__ __forceinline__ void st(uint32_t a, const uint32_t* r) {
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-                     :: "r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-    }
-};
-template <> struct GxSt<16> {
-    static __device__ __forceinline__ void st(uint32_t a, const uint32_t* r) {
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                     :: "r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-    }
-};
-template <> struct GxSt<32> {
-    static __device__ __forceinline__ void st(uint32_t a, const uint32_t* r) {
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-                     "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-                     :: "r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
-                        "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
-                        "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
-    }
-};
-
-template <int NT>
+template <bool TABLE, int TA, bool DUAL, int NBLK>
 __global__ void __launch_bounds__(GX_THREADS, 1)
-k_gemm_mxf4(const __grid_constant__ GxParams p, const __grid_constant__ CUtensorMap map_x,
-            const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s) {
-    constexpr int CB = NT / 32;                    // TMEM columns the activation scales of one 64-k block fill
-    constexpr int CBS = CB < 4 ? 4 : CB;           // ... and the columns between two blocks (scale addresses stay multiples of 4)
-    constexpr int SLOT = 16 + 4 * CBS;             // TMEM columns of one step's scales
-    constexpr uint32_t B_BYTES = NT * 128u;
+k_gemm_mxf4(const __grid_constant__ GxParams p, const __grid_constant__ GxMaps maps) {
+    static_assert(!DUAL || TA == 2, "a dual item is one gate and one up tile");
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ uint64_t full_bar[GX_MAX_STEPS], sf_bar[GX_MAX_STEPS], empty_bar[GX_MAX_STEPS], slab_bar[GX_MAX_SLABS], done_bar;
+    __shared__ uint64_t full_bar[GX_MAX_STAGES], empty_bar[GX_MAX_STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base_s;
-    __shared__ float sx[NT];                       // 1 / (gs_w * gs_x[token]) of the job's rows
+    __shared__ float sx[2][DUAL ? 2 : 1][GX_MAX_NT];   // 1 / (gs_w * gs_x[token]) of an item's tokens, double-buffered
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int K = p.K, nst = K >> 8, R = p.R;
-
-    GxJob J;
-    const int chunk = (int)blockIdx.x / p.n_jobs, ji = (int)blockIdx.x - chunk * p.n_jobs;
-    const void* mw = &map_w;
-    const void* ms = &map_s;
-    if (p.table) {
-        pdl_wait();                                // the table is written by an earlier kernel of the stream
-        J = p.table[ji];
-        if (J.rows <= 0) return;                   // an unused slot: the whole CTA leaves before it owns anything
-        mw = J.mw; ms = J.ms;
-    } else {
-        J = p.one;
-        J.row0 = ji * NT;
-        J.rows = min(NT, J.rows - J.row0);
-        J.y += (size_t)J.row0 * J.ldy;
-        J.gs_x += J.row0;
-    }
-    // Jobs of a table launch with few rows load (and multiply) only a 32- or 64-row box of activations: an
-    // expert that three tokens chose should not pull a 128-row tile through L2 at every step.  In table
-    // mode the two weight-map parameters are unused and carry the activation maps with the smaller boxes.
-    int nb = NT;
-    const void* mx = &map_x;
-    if (p.table) {
-        if (NT > 32 && J.rows <= 32) { nb = 32; mx = &map_w; }
-        else if (NT > 64 && J.rows <= 64) { nb = 64; mx = &map_s; }
-    }
-    // this CTA's consecutive tiles of R weight rows: [tile0, tile0 + ntile)
-    const int tile0 = chunk * p.T, ntile = min(p.T, (J.N + R - 1) / R - tile0);
-    if (ntile <= 0) return;
-    const int nsteps = ntile * nst;                // step g: tile g / nst, 256-k block g % nst
-    const int sps = p.sps;                         // steps one scale slab covers; slab j = steps [j * sps, (j + 1) * sps)
-    const uint32_t slab_bytes = (uint32_t)R * (uint32_t)p.sc_box;
-
-    unsigned char* ringA = smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);  // sa slots of packed weights
-    unsigned char* ringB = ringA + (size_t)p.sa * p.a_slot;                     // sb slots of packed activations
-    unsigned char* scl = ringB + (size_t)p.sb * B_BYTES;                        // ring of weight-scale slabs [R x sc_box], 1 KB aligned (swizzle)
-    unsigned char* sfbs = scl + (size_t)p.nslot * slab_bytes;                   // per activation slot NT x 16 B of activation scales
+    const int K = p.K, nst = K >> 8, R = p.R, NT = p.NT, S = p.stages;
+    constexpr int CBS = 4 * NBLK, SLOT = 16 * TA + 4 * CBS;
+    const int col_sf = p.nbuf * TA * NT;
+    const int nrow = DUAL ? R : TA * R;                 // weight rows of each matrix an item covers
 
     pdl_launch_dependents();
-    if (warp >= 4) {
-        const int i = tid - 128;
-        if (i < nsteps) mbar_init(smem_u32(&full_bar[i]), 1);
-        else if (i >= 64 && i < 64 + nsteps) mbar_init(smem_u32(&sf_bar[i - 64]), 128);
-        else if (i >= 128 && i < 128 + nsteps) mbar_init(smem_u32(&empty_bar[i - 128]), 1);
-        else if (i >= 192 && i < 192 + GX_MAX_SLABS) mbar_init(smem_u32(&slab_bar[i - 192]), 1);
-        else if (i == 255) mbar_init(smem_u32(&done_bar), p.nacc >= 2 ? 2 : 1);
-        mbar_fence_init();
-    }
     if (warp == 2) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&tmem_base_s)), "r"(GX_TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    } else if (warp == 1) {
+        if (lane < S) {
+            mbar_init(smem_u32(&full_bar[lane]), 2 + TA);  // the two TMA warps, one scale warp per weight tile
+            mbar_init(smem_u32(&empty_bar[lane]), 1);
+        }
+        if (lane < 2) { mbar_init(smem_u32(&acc_full[lane]), 1); mbar_init(smem_u32(&acc_empty[lane]), 8); }
+        mbar_fence_init();
     }
     gx_fence_before();
     __syncthreads();
     gx_fence_after();
     const uint32_t tmem = tmem_base_s;
+    if (TABLE) pdl_wait();                             // the table is written by an earlier kernel of the stream
+    const int total = (TABLE ? *p.n_jobs_dev : p.n_jobs) * p.tiles, first = blockIdx.x, stride = gridDim.x;
+    const int n_items = first < total ? (total - first + stride - 1) / stride : 0;
+
+    unsigned char* ringA = smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);
+    const uint32_t ring0 = smem_u32(ringA);
+    const uint32_t full0 = smem_u32(&full_bar[0]), empty0 = smem_u32(&empty_bar[0]);
 
     if (warp == 0) {
-        // ---- TMA producer: lane l issues steps l, l + 32, .. (and the scale slab that starts with such a step) ----
-        if (lane == 0) {
-            asm volatile("prefetch.tensormap [%0];" :: "l"(mw) : "memory");
-            asm volatile("prefetch.tensormap [%0];" :: "l"(ms) : "memory");
-            asm volatile("prefetch.tensormap [%0];" :: "l"(mx) : "memory");
-        }
-        if (!p.prefetch_before_wait) pdl_wait();
-        const uint32_t full0 = smem_u32(&full_bar[0]), empty0 = smem_u32(&empty_bar[0]), slab0 = smem_u32(&slab_bar[0]);
-        const uint32_t step_bytes = (uint32_t)R * 128u + (uint32_t)nb * 128u + (uint32_t)nb * 16u;
-        int t = lane / nst, it = lane - t * nst;
-        const int spt = nst / sps;                 // slabs per tile
-        for (int g = lane; g < nsteps; g += 32) {
-            const int rown0 = (tile0 + t) * R;
-            const int js = p.sc_swz ? (it >> 3) : 0;                 // slab of this step within its tile
-            if ((p.sc_swz ? (it & 7) : it) == 0) {
-                // the slab of scale rows that steps [g, g + sps) read; its slot is free once the MMAs of the
-                // last step of the slab that held it have completed (their scale movers are then done as well)
-                const int j = t * spt + js;
-                if (j >= p.nslot) mbar_wait_spin(empty0 + ((j - p.nslot + 1) * sps - 1) * 8, 0, p.status, 8);
-                mbar_expect_tx(slab0 + j * 8, slab_bytes);
-                gx_tma_2d(smem_u32(scl) + (uint32_t)(j % p.nslot) * slab_bytes, ms, js * p.sc_box, rown0, slab0 + j * 8);
-            }
-            // The weights stream from HBM and get the deep ring; the activations come from L2 and share a
-            // short ring with the step's scale slot in TMEM.  Both loads of a step signal one barrier.
-            const int sA = g % p.sa, sB = g % p.sb;
-            if (g >= p.sa) mbar_wait_spin(empty0 + (g - p.sa) * 8, 0, p.status, 9);
-            const uint32_t bar = full0 + g * 8;
-            mbar_expect_tx(bar, step_bytes);
-            gx_tma_2d(smem_u32(ringA) + (uint32_t)sA * p.a_slot, mw, it * 128, rown0, bar);     // weights may be read early (stable weights)
-            pdl_wait();                                                           // the activations come from the quantiser launch
-            if (g >= p.sb) mbar_wait_spin(empty0 + (g - p.sb) * 8, 0, p.status, 7);
-            gx_tma_2d(smem_u32(ringB) + (uint32_t)sB * B_BYTES, mx, it * 128, J.row0, bar);
-            bulk_g2s(smem_u32(sfbs) + (uint32_t)sB * NT * 16u, p.sfb + ((size_t)it * p.sfb_rows + (size_t)J.row0) * 16, (uint32_t)nb * 16u, bar);
-            it += 32; while (it >= nst) { it -= nst; ++t; }
-        }
-        __syncwarp();
-        // The tcgen05.commit arrivals on empty_bar are asynchronous: wait for the last one of every
-        // stage, or the CTA could exit with an arrival in flight that lands in the next CTA's shared memory.
-        for (int g = max(0, nsteps - p.sa) + lane; g < nsteps; g += 32)
-            mbar_wait_spin(empty0 + g * 8, 0, p.status, 10);
-        __syncwarp();
-    } else if (warp == 1 || (warp == 3 && p.nacc >= 2)) {
-        // ---- MMA issuers: the whole warp walks the loop, lane 0 issues ----
-        // A chain of MMAs into one accumulator runs at the latency of an MMA, not at its issue rate, and
-        // that latency (about 110 cycles) exceeds the execution time of an MMA narrower than 256 columns.
-        // So a tile has nacc accumulators -- k-block `it` adds into accumulator it % nacc, the epilogue adds
-        // them up in a fixed order -- and with two or more of them two warps issue: warp 1 the even
-        // k-blocks, warp 3 the odd ones (different accumulators, so no order between the warps matters).
-        const int mwi = warp == 1 ? 0 : 1, two = p.nacc >= 2;
-        const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(nb >> 3) << 17) | ((128u >> 4) << 24);
-        const uint64_t dA0 = gx_desc(smem_u32(ringA)), dB0 = gx_desc(smem_u32(ringB));
-        const uint32_t sf0 = smem_u32(&sf_bar[0]), empty0 = smem_u32(&empty_bar[0]);
-        int sA = 0, sB = 0, sF = 0, t = 0, it = 0;
-        for (int g = 0; g < nsteps; ++g) {
-            if (!two || (it & 1) == mwi) {
-                mbar_wait_spin(sf0 + g * 8, 0, p.status, 11);
-                gx_fence_after();
-                if (lane == 0) {
-                    const uint32_t slot = tmem + GX_COL_SF + (uint32_t)sF * SLOT;
-                    const uint64_t soA = (uint64_t)(((uint32_t)sA * p.a_slot) >> 4), soB = (uint64_t)(((uint32_t)sB * B_BYTES) >> 4);
-                    const uint32_t tD = tmem + (uint32_t)((t * p.nacc + (it & (p.nacc - 1))) * NT);
-                    const uint32_t first = it < p.nacc ? 0u : 1u;           // the first k-block of an accumulator starts it
-                    #pragma unroll
-                    for (int kb = 0; kb < 4; ++kb) {
-                        asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                                     " tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%5], [%6], p;\n}"
-                                     :: "r"(tD), "l"(dA0 + soA + kb * 2), "l"(dB0 + soB + kb * 2), "r"(idesc),
-                                        "r"(kb ? 1u : first), "r"(slot + kb * 4), "r"(slot + 16 + kb * CBS) : "memory");
-                    }
-                    gx_commit(empty0 + g * 8);
+        // ---- TMA: packed weights.  The whole warp walks the loop and waits, one lane issues. ----
+        if (!TABLE && !p.prefetch_before_wait) pdl_wait();
+        const uint32_t bytes = (uint32_t)(TA * R) * 128u;
+        int s = 0; uint32_t ph = 1;
+        for (int i = 0; i < n_items; ++i) {
+            const GxItem q = gx_item<TABLE>(p, first + i * stride);
+            const void* mw = TABLE ? p.table[q.job].mw : (const void*)&maps.w;
+            const void* mw2 = DUAL ? p.table[q.job].mw2 : mw;
+            const int r0 = q.tile * nrow;
+            for (int it = 0; it < nst; ++it) {
+                mbar_wait_spin(empty0 + s * 8, ph, p.status, 9);
+                if (elect_one()) {
+                    const uint32_t bar = full0 + s * 8, dst = ring0 + (uint32_t)(s * TA) * p.a_slot;
+                    mbar_expect_tx(bar, bytes);
+                    gx_tma_2d(dst, mw, it * 128, r0, bar);
+                    if (TA == 2) gx_tma_2d(dst + p.a_slot, mw2, it * 128, DUAL ? r0 : r0 + R, bar);
                 }
                 __syncwarp();
+                if (++s == S) { s = 0; ph ^= 1; }
             }
-            if (++sA == p.sa) sA = 0;
-            if (++sB == p.sb) sB = 0;
-            if (++sF == p.ssf) sF = 0;
-            if (++it == nst) { it = 0; ++t; }
         }
-        if (lane == 0) gx_commit(smem_u32(&done_bar));
-        __syncwarp();
-    } else if (warp >= 4) {
-        // ---- scale movers, then epilogue ----
-        const int tm = tid - 128, grp = tm >> 7, q4 = warp & 3;
+        // The commits that free the stages arrive asynchronously: wait for the last one of every stage, or it could
+        // land in the shared memory of the next CTA on this SM.
+        for (int k = 0; k < S; ++k) {
+            mbar_wait_spin(empty0 + s * 8, ph, p.status, 10);
+            if (++s == S) { s = 0; ph ^= 1; }
+        }
+    } else if (warp == 3) {
+        // ---- TMA: packed activations and their scales ----
+        if (!TABLE) pdl_wait();                        // they come from the quantiser launch
+        int s = 0; uint32_t ph = 1;
+        constexpr uint32_t sfb_step = NBLK * 2048u;
+        for (int i = 0; i < n_items; ++i) {
+            const GxJob J = gx_job<TABLE>(p, gx_item<TABLE>(p, first + i * stride).job);
+            // jobs of a table with few rows load a small box: an expert that three tokens chose should not pull
+            // a whole activation tile through L2 at every step
+            int nb = NT; const void* mx = &maps.x[0];
+            if (TABLE) {
+                if (J.rows <= 16) { nb = 16; mx = &maps.x[3]; }
+                else if (NT > 32 && J.rows <= 32) { nb = 32; mx = &maps.x[2]; }
+                else if (NT > 64 && J.rows <= 64) { nb = 64; mx = &maps.x[1]; }
+            }
+            const unsigned char* sf = J.sfb;
+            for (int it = 0; it < nst; ++it) {
+                mbar_wait_spin(empty0 + s * 8, ph, p.status, 7);
+                if (elect_one()) {
+                    const uint32_t bar = full0 + s * 8;
+                    mbar_expect_tx(bar, (uint32_t)nb * 128u + sfb_step);
+                    gx_tma_2d(ring0 + p.b_off + (uint32_t)s * (uint32_t)NT * 128u, mx, it * 128, J.row0, bar);
+                    bulk_g2s(ring0 + p.sf_off + (uint32_t)s * sfb_step, sf, sfb_step, bar);
+                }
+                sf += sfb_step;
+                __syncwarp();
+                if (++s == S) { s = 0; ph ^= 1; }
+            }
+        }
+    } else if (warp == 1) {
+        // ---- MMA issuer ----
+        const uint64_t dA0 = gx_desc(ring0), dB0 = gx_desc(ring0 + p.b_off);
+        const uint64_t dTS0 = gx_desc_sf(ring0 + p.ts_off), dSF0 = gx_desc_sf(ring0 + p.sf_off);
+        int s = 0, sf = 0, ps = 0; uint32_t ph = 0, pph = 0;      // stage and phase; scale slot; stage and phase of the step that had the slot last
+        int g = 0;
+        for (int i = 0; i < n_items; ++i) {
+            int n = NT;
+            if (TABLE) n = min(NT, (p.table[gx_item<TABLE>(p, first + i * stride).job].rows + 15) & ~15);
+            const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24);
+            const int buf = p.nbuf == 2 ? (i & 1) : 0, use = p.nbuf == 2 ? (i >> 1) : i;
+            if (use > 0) mbar_wait_spin(smem_u32(&acc_empty[buf]), (use - 1) & 1, p.status, 14);
+            const uint32_t tD = tmem + (uint32_t)(buf * TA * NT);
+            for (int it = 0; it < nst; ++it, ++g) {
+                mbar_wait_spin(full0 + s * 8, ph, p.status, 11);
+                if (g >= p.nslot) {                    // the slot's last reader is done
+                    mbar_wait_spin(empty0 + ps * 8, pph, p.status, 6);
+                    if (++ps == S) { ps = 0; pph ^= 1; }
+                }
+                gx_fence_after();
+                if (elect_one()) {
+                    const uint32_t slot = tmem + (uint32_t)(col_sf + sf * SLOT);
+                    #pragma unroll
+                    for (int kb = 0; kb < 4; ++kb) {
+                        #pragma unroll
+                        for (int t = 0; t < TA; ++t)
+                            gx_cp_sf(slot + t * 16 + kb * 4, dTS0 + (uint64_t)((s * TA + t) * 128 + kb * 32));
+                        #pragma unroll                // (a loop with a count from memory in here cost 0.4 us per step)
+                        for (int b = 0; b < NBLK; ++b)
+                            gx_cp_sf(slot + 16 * TA + kb * CBS + 4 * b, dSF0 + (uint64_t)((s * NBLK + b) * 128 + kb * 32));
+                    }
+                    const uint64_t dB = dB0 + (uint64_t)(((uint32_t)s * (uint32_t)NT * 128u) >> 4);
+                    #pragma unroll
+                    for (int t = 0; t < TA; ++t) {
+                        const uint64_t dA = dA0 + (uint64_t)(((uint32_t)(s * TA + t) * p.a_slot) >> 4);
+                        #pragma unroll
+                        for (int kb = 0; kb < 4; ++kb)
+                            asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                                         " tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%5], [%6], p;\n}"
+                                         :: "r"(tD + (uint32_t)(t * NT)), "l"(dA + kb * 2), "l"(dB + kb * 2), "r"(idesc),
+                                            "r"((uint32_t)(it | kb)), "r"(slot + t * 16 + kb * 4), "r"(slot + 16 * TA + kb * CBS) : "memory");
+                    }
+                    gx_commit(empty0 + s * 8);
+                    if (it == nst - 1) gx_commit(smem_u32(&acc_full[buf]));
+                }
+                __syncwarp();
+                if (++s == S) { s = 0; ph ^= 1; }
+                if (++sf == p.nslot) sf = 0;
+            }
+        }
+    } else if (warp >= 4 && warp < 8) {
+        // ---- weight scales.  A unit is two steps of one weight tile; warp w takes every NW-th unit. ----
+        // NW keeps a warp's consecutive units at most S steps apart: a warp sees only its own uses of a stage, and further
+        // apart it could ask for a phase of empty_bar whose predecessor has not completed either (a parity cannot tell).
+        const int NW = TA == 2 ? (S >= 4 ? 4 : 2) : max(1, min(4, S >> 1));
+        if (!TABLE && !p.prefetch_before_wait) pdl_wait();
+        const int pairs = (nst + 1) >> 1, upi = pairs * TA;
+        const size_t pitch = (size_t)(K >> 4);
+        const unsigned char* scp[TA];                  // of item ci: the tile's first scale row
+        int ci = -1, rows_t[TA];
+        auto load = [&](int i, int u, uint4 (&v)[2][4]) {
+            if (i != ci) {
+                ci = i;
+                const GxItem q = gx_item<TABLE>(p, first + i * stride);
+                #pragma unroll
+                for (int t = 0; t < TA; ++t) {
+                    const unsigned char* sc = TABLE ? (DUAL && t ? p.table[q.job].sc2 : p.table[q.job].sc) : p.one.sc;
+                    const int N = TABLE ? p.table[q.job].N : p.one.N, r0 = q.tile * nrow + (DUAL ? 0 : t * R);
+                    scp[t] = sc + (size_t)r0 * pitch;
+                    rows_t[t] = min(R, N - r0);
+                    // the tile's scale rows, asked into L2 by one warp
+                    if (warp == 4 + t)
+                        for (int r = lane; r < rows_t[t]; r += 32)
+                            for (size_t o = 0; o < pitch; o += 128)
+                                asm volatile("prefetch.global.L2 [%0];" :: "l"(scp[t] + (size_t)r * pitch + o));
+                }
+            }
+            const int t = TA == 2 ? (u & 1) : 0, st = (TA == 2 ? u >> 1 : u) * 2;
+            const unsigned char* base = (TA == 2 && t ? scp[TA - 1] : scp[0]) + (size_t)st * 16;
+            const int rv = TA == 2 && t ? rows_t[TA - 1] : rows_t[0];
+            #pragma unroll
+            for (int h = 0; h < 2; ++h)
+                #pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int r = lane + 32 * c;
+                    v[h][c] = (r < rv && st + h < nst) ? __ldg(reinterpret_cast<const uint4*>(base + (size_t)r * pitch + h * 16)) : make_uint4(0u, 0u, 0u, 0u);
+                }
+        };
+        int i = 0, u = warp - 4;
+        auto settle = [&] { while (u >= upi) { u -= upi; ++i; } };
+        uint4 v[2][4];
+        if (u >= NW) i = n_items;                       // an idle warp
+        settle();
+        if (i < n_items) load(i, u, v);
+        while (i < n_items) {
+            const int g0 = i * nst + (TA == 2 ? u >> 1 : u) * 2, t = TA == 2 ? (u & 1) : 0;
+            const int left = (i + 1) * nst - g0;       // steps of the item from this one on
+            uint4 cur[2][4];
+            #pragma unroll
+            for (int h = 0; h < 2; ++h)
+                #pragma unroll
+                for (int c = 0; c < 4; ++c) cur[h][c] = v[h][c];
+            u += NW; settle();
+            if (i < n_items) load(i, u, v);
+            #pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (h >= left) break;
+                const int g = g0 + h, use = g / S, s = g - use * S;
+                mbar_wait_spin(empty0 + s * 8, (use & 1) ^ 1, p.status, 13);
+                uint4* o = reinterpret_cast<uint4*>(ringA + p.ts_off + (size_t)(s * TA + t) * 2048) + lane;
+                o[0] = make_uint4(cur[h][0].x, cur[h][1].x, cur[h][2].x, cur[h][3].x);
+                o[32] = make_uint4(cur[h][0].y, cur[h][1].y, cur[h][2].y, cur[h][3].y);
+                o[64] = make_uint4(cur[h][0].z, cur[h][1].z, cur[h][2].z, cur[h][3].z);
+                o[96] = make_uint4(cur[h][0].w, cur[h][1].w, cur[h][2].w, cur[h][3].w);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // generic-proxy stores -> the copy's async-proxy reads
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full0 + s * 8);
+            }
+        }
+    } else if (warp >= 8) {
+        // ---- epilogue: two groups of four warps (one per TMEM lane quadrant) take alternate 16-token chunks ----
+        const int te = tid - 256, grp = te >> 7, q4 = warp & 3, r = q4 * 32 + lane;
         const uint32_t tq = tmem + ((uint32_t)(q4 * 32) << 16);
-        pdl_wait();
-        if (tm < NT) sx[tm] = tm < J.rows ? 1.0f / (J.gs_w[0] * J.gs_x[tm]) : 0.f;
-        named_sync(1, GX_MOVERS);
-        const uint32_t full0 = smem_u32(&full_bar[0]), sf0 = smem_u32(&sf_bar[0]), slab0 = smem_u32(&slab_bar[0]);
-        const uint32_t empty0 = smem_u32(&empty_bar[0]);
-        int s = grp % p.sb, sf = grp % p.ssf;
-        int t = grp / nst, it = grp - t * nst;
-        const int spt = nst / sps;
-        for (int g = grp; g < nsteps; g += 2) {
-            const int js = p.sc_swz ? (it >> 3) : 0, is = p.sc_swz ? (it & 7) : it;     // slab within the tile, step within the slab
-            const int j = t * spt + js, valid = J.N - (tile0 + t) * R;    // weight rows of this tile that exist (may exceed R)
-            mbar_wait_spin(slab0 + j * 8, 0, p.status, 12);
-            mbar_wait_spin(full0 + g * 8, 0, p.status, 13);
-            // the scale slot in TMEM is free once the MMAs of the step that used it last have completed
-            // (implied by full[g] when there are as many slots as activation slots)
-            if (p.ssf < p.sb && g >= p.ssf) mbar_wait_spin(empty0 + (g - p.ssf) * 8, 0, p.status, 6);
-            // weights: lane l holds rows l, l+32, l+64, l+96, 16 bytes each = four 64-k blocks x four scales;
-            // block kb of row 32c + l goes to column kb*4 + c
-            const unsigned char* sl = scl + (size_t)(j % p.nslot) * slab_bytes;
-            uint32_t ra[16];
-            #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int r = lane + 32 * c;
-                uint32_t off;
-                if (p.sc_swz) off = (uint32_t)r * 128u + (uint32_t)((is ^ (r & 7)) << 4);
-                else off = (uint32_t)r * (uint32_t)p.sc_box + (uint32_t)is * 16u;
-                const uint4 v = (r < R && r < valid) ? *reinterpret_cast<const uint4*>(sl + off) : make_uint4(0u, 0u, 0u, 0u);
-                ra[c] = v.x; ra[4 + c] = v.y; ra[8 + c] = v.z; ra[12 + c] = v.w;
+        if (!TABLE) pdl_wait();
+        for (int i = 0; i < n_items; ++i) {
+            const GxItem q = gx_item<TABLE>(p, first + i * stride);
+            const GxJob J = gx_job<TABLE>(p, q.job);
+            const int buf = p.nbuf == 2 ? (i & 1) : 0, use = p.nbuf == 2 ? (i >> 1) : i;
+            float (*f)[GX_MAX_NT] = sx[i & 1];
+            if (te < J.rows) {
+                const float gx = J.gs_x[te];
+                f[0][te] = 1.0f / (J.gs_w[0] * gx);
+                if (DUAL) f[DUAL ? 1 : 0][te] = 1.0f / (J.gs_w2[0] * gx);
             }
-            // activations: lane l holds tokens l, l+32, ..; block kb of token 32c + l goes to column 16 + kb*CBS + c
-            uint32_t rb[4 * CBS];
-            const unsigned char* sb = sfbs + (size_t)s * NT * 16;
+            named_sync(1, 256);
+            mbar_wait_spin(smem_u32(&acc_full[buf]), use & 1, p.status, 14);
+            gx_fence_after();
+            const int row = q.tile * nrow + r;
+            bool ok[TA];                               // this lane's weight row of each tile exists
             #pragma unroll
-            for (int c = 0; c < CBS; ++c) {
-                const uint4 v = (c < CB && 32 * c < nb) ? *reinterpret_cast<const uint4*>(sb + (size_t)(lane + 32 * c) * 16) : make_uint4(0u, 0u, 0u, 0u);
-                rb[c] = v.x; rb[CBS + c] = v.y; rb[2 * CBS + c] = v.z; rb[3 * CBS + c] = v.w;
+            for (int t = 0; t < TA; ++t) ok[t] = r < R && row + (DUAL ? 0 : t * R) < J.N;
+            for (int c0 = grp * 16; c0 < J.rows; c0 += 32) {
+                float d[TA][16];
+                #pragma unroll
+                for (int t = 0; t < TA; ++t) gx_ld16(tq + (uint32_t)((buf * TA + t) * NT + c0), d[t]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                #pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    if (DUAL) {
+                        const float ga = fminf(d[0][j] * f[0][c0 + j], p.limit);
+                        const float ua = fminf(fmaxf(d[TA - 1][j] * f[DUAL ? 1 : 0][c0 + j], -p.limit), p.limit);
+                        d[0][j] = (ga / (1.f + __expf(-ga))) * ua;
+                    } else {
+                        #pragma unroll
+                        for (int t = 0; t < TA; ++t) d[t][j] *= f[0][c0 + j];
+                    }
+                }
+                const int left = J.rows - c0;
+                #pragma unroll
+                for (int t = 0; t < (DUAL ? 1 : TA); ++t) {
+                    float* y = J.y + (size_t)c0 * J.ldy + row + t * R;
+                    if (ok[t]) {
+                        if (left >= 16) {
+                            #pragma unroll
+                            for (int j = 0; j < 16; ++j, y += J.ldy) *y = d[t][j];
+                        } else {
+                            #pragma unroll
+                            for (int j = 0; j < 16; ++j, y += J.ldy) if (j < left) *y = d[t][j];
+                        }
+                    }
+                }
             }
-            const uint32_t slot = tq + GX_COL_SF + (uint32_t)sf * SLOT;
-            GxSt<16>::st(slot, ra);
-            GxSt<4 * CBS>::st(slot + 16, rb);
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             gx_fence_before();
-            mbar_arrive(sf0 + g * 8);
-            s += 2; while (s >= p.sb) s -= p.sb;
-            sf += 2; while (sf >= p.ssf) sf -= p.ssf;
-            it += 2; while (it >= nst) { it -= nst; ++t; }
-        }
-        // epilogue: group grp takes columns [grp * NT/2, (grp + 1) * NT/2) of every tile
-        mbar_wait_spin(smem_u32(&done_bar), 0, p.status, 14);
-        gx_fence_after();
-        const int r = q4 * 32 + lane;
-        #pragma unroll 1
-        for (int te = 0; te < ntile; ++te) {
-            const int row = (tile0 + te) * R + r;
-            const bool ok = r < R && row < J.N;
-            #pragma unroll 1
-            for (int c0 = grp * (NT / 2); c0 < (grp + 1) * (NT / 2); c0 += 16) {
-                if (c0 >= J.rows) break;             // warp-uniform: the remaining tokens do not exist
-                float d[16];
-                #pragma unroll 1
-                for (int a = 0; a < p.nacc; ++a) {
-                    uint32_t v[16];
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                                 : "r"(tq + (uint32_t)((te * p.nacc + a) * NT + c0)));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    #pragma unroll
-                    for (int j = 0; j < 16; ++j) d[j] = a == 0 ? __uint_as_float(v[j]) : d[j] + __uint_as_float(v[j]);     // accumulators in index order
-                    if (a + 1 < p.nacc && (a + 1) >= nst) break;     // fewer k-blocks than accumulators: the rest were never started
-                }
-                if (ok) {
-                    #pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        if (c0 + j < J.rows) J.y[(size_t)(c0 + j) * J.ldy + row] = d[j] * sx[c0 + j];
-                }
-            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&acc_empty[buf]));
         }
     }
     gx_fence_before();
@@ -345,93 +380,116 @@ k_gemm_mxf4(const __grid_constant__ GxParams p, const __grid_constant__ CUtensor
 }
 
 // ---- per-token activation quantiser -------------------------------------------------------------
-// One CTA per activation row.  MODE 0: bf16 rows; 1: f32 rows; 2: f32 rows of the clamped SwiGLU
-// silu(min(g, limit)) * clamp(u, -limit, limit) of two product vectors (the MoE down projection's input).
-// src_row != nullptr: output row r is input row src_row[r] (gathers token rows into expert order).
-// Output: packed [*, K/2] codes, scales step-major [K/256][sfb_rows][16], gsx[r] = 2688 / amax(row r).
-// Rows in [M, rows_total) only get zero scales (they pad the last tile of a dense call).
-template <int MODE>
-__global__ void __launch_bounds__(256)
-k_quant_act(const void* __restrict__ xin, const void* __restrict__ xin2, float limit, const int* __restrict__ src_row,
-            const int* __restrict__ m_dev, int M, int K, unsigned char* __restrict__ xq, unsigned char* __restrict__ sfb,
-            size_t sfb_rows, float* __restrict__ gsx) {
-    __shared__ uint32_t red[8];
+// One CTA per activation row (bf16 or f32), which is read once and kept in registers for rows of up to 2 * THREADS
+// groups of 16.  CP: output in the order of ActQuant, to every destination of the row (a token that nine experts
+// read is quantised once and written nine times); otherwise packed [M, K/2] and scales step-major [K/256][M][16].
+template <bool F32, bool CP, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+k_quant_act(const void* __restrict__ xin, int M, int K, const __grid_constant__ ActQuant q) {
+    constexpr int KEEP = 2;
+    __shared__ uint32_t red[THREADS / 32];
     const int row = blockIdx.x, tid = threadIdx.x, groups = K >> 4;
     pdl_launch_dependents();
     pdl_wait();
-    if (m_dev) M = m_dev[0];                        // row count decided on the device (rows grouped by expert)
-    if (row >= M) {
-        if (m_dev) return;
-        for (int st = tid; st < (K >> 8); st += 256)
-            *reinterpret_cast<uint4*>(sfb + ((size_t)st * sfb_rows + row) * 16) = make_uint4(0u, 0u, 0u, 0u);
-        return;
-    }
-    const size_t src = src_row ? (size_t)src_row[row] : (size_t)row;
-    auto load = [&](int g, float (&v)[16]) {
-        if (MODE == 0) {
-            const uint4* r = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(xin) + src * K) + 2 * g;
-            const uint4 a = r[0], b = r[1];
-            const uint32_t u[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-            #pragma unroll
-            for (int j = 0; j < 8; ++j) { v[2 * j] = __uint_as_float(u[j] << 16); v[2 * j + 1] = __uint_as_float(u[j] & 0xffff0000u); }
-        } else {
-            const float4* r = reinterpret_cast<const float4*>(static_cast<const float*>(xin) + src * K) + 4 * g;
-            const float4* r2 = MODE == 2 ? reinterpret_cast<const float4*>(static_cast<const float*>(xin2) + src * K) + 4 * g : nullptr;
-            #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                float4 a = r[q];
-                if (MODE == 2) {
-                    const float4 u = r2[q];
-                    const float gg[4] = {fminf(a.x, limit), fminf(a.y, limit), fminf(a.z, limit), fminf(a.w, limit)};
-                    const float uu[4] = {fminf(fmaxf(u.x, -limit), limit), fminf(fmaxf(u.y, -limit), limit),
-                                         fminf(fmaxf(u.z, -limit), limit), fminf(fmaxf(u.w, -limit), limit)};
-                    a = make_float4((gg[0] / (1.f + __expf(-gg[0]))) * uu[0], (gg[1] / (1.f + __expf(-gg[1]))) * uu[1],
-                                    (gg[2] / (1.f + __expf(-gg[2]))) * uu[2], (gg[3] / (1.f + __expf(-gg[3]))) * uu[3]);
-                }
-                v[4 * q] = a.x; v[4 * q + 1] = a.y; v[4 * q + 2] = a.z; v[4 * q + 3] = a.w;
-            }
-        }
+    // eight words of a group: bf16 pairs as they lie in memory, or the sixteen floats
+    struct Grp { uint32_t u[F32 ? 16 : 8]; };
+    auto load = [&](int g, Grp& v) {
+        const uint4* r = reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(xin) + (size_t)row * K * (F32 ? 4 : 2)) + (size_t)g * (F32 ? 4 : 2);
+        #pragma unroll
+        for (int k = 0; k < (F32 ? 4 : 2); ++k) { const uint4 a = r[k]; v.u[4 * k] = a.x; v.u[4 * k + 1] = a.y; v.u[4 * k + 2] = a.z; v.u[4 * k + 3] = a.w; }
     };
-    float first[16];
     // maximum over the bit patterns of |x| (they order like the values; an infinity or a NaN wins instead of
     // being dropped): a row that holds one gets a NaN global scale, and with it NaN outputs
     uint32_t ai = 0u;
-    for (int g = tid; g < groups; g += 256) {
-        float v[16];
-        load(g, v);
+    auto fold = [&](const Grp& v) {
         #pragma unroll
-        for (int j = 0; j < 16; ++j) { ai = max(ai, __float_as_uint(v[j]) & 0x7fffffffu); if (g == tid) first[j] = v[j]; }
-    }
+        for (int j = 0; j < (F32 ? 16 : 8); ++j) {
+            if (F32) ai = max(ai, v.u[j] & 0x7fffffffu);
+            else ai = max(ai, max((v.u[j] << 16) & 0x7fffffffu, v.u[j] & 0x7fff0000u));
+        }
+    };
+    Grp keep[KEEP];
     #pragma unroll
-    for (int o = 16; o; o >>= 1) ai = max(ai, __shfl_xor_sync(0xffffffffu, ai, o));
+    for (int k = 0; k < KEEP; ++k) if (tid + k * THREADS < groups) load(tid + k * THREADS, keep[k]);
+    #pragma unroll
+    for (int k = 0; k < KEEP; ++k) if (tid + k * THREADS < groups) fold(keep[k]);
+    for (int g = tid + KEEP * THREADS; g < groups; g += THREADS) { Grp v; load(g, v); fold(v); }
+    ai = __reduce_max_sync(0xffffffffu, ai);
     if ((tid & 31) == 0) red[tid >> 5] = ai;
     __syncthreads();
     ai = red[0];
     #pragma unroll
-    for (int w = 1; w < 8; ++w) ai = max(ai, red[w]);
+    for (int w = 1; w < THREADS / 32; ++w) ai = max(ai, red[w]);
     const float gs = ai >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : nvfp4_global_scale(__uint_as_float(ai));
-    if (tid == 0) gsx[row] = gs;
-    for (int g = tid; g < groups; g += 256) {
-        float v[16];
-        if (g == tid) {
-            #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = first[j];
-        } else load(g, v);
+    const int nst = K >> 8, ndst = CP ? q.ndst : 1;
+    // destination d of this row: packed row, and where its column of the scale blocks starts
+    auto dst_row = [&](int d) { return q.pos ? q.pos[(size_t)row * ndst + d] : row; };
+    auto dst_sf = [&](int d) -> size_t {
+        int job, c;
+        if (q.sfrow) { const int s = q.sfrow[(size_t)row * ndst + d], w = q.nblk * 128; job = s / w; c = s - job * w; }
+        else { job = row / q.NT; c = row - job * q.NT; }
+        return ((size_t)job * nst * q.nblk + (c >> 7)) * 2048 + (size_t)((c & 31) * 16 + ((c & 127) >> 5) * 4);
+    };
+    if (CP) { if (tid < ndst) q.gsx[dst_row(tid)] = gs; }
+    else if (tid == 0) q.gsx[row] = gs;
+    auto emit = [&](int g, const Grp& v) {
         uint32_t lo, hi; int code;
-        quantize_group(v, gs, lo, hi, code);
-        reinterpret_cast<uint2*>(xq + (size_t)row * (K >> 1))[g] = make_uint2(lo, hi);
-        sfb[((size_t)(g >> 4) * sfb_rows + row) * 16 + (g & 15)] = (unsigned char)code;
-    }
+        if constexpr (F32) {
+            float f[16];
+            #pragma unroll
+            for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(v.u[j]);
+            quantize_group(f, gs, lo, hi, code);
+        } else {
+            quantize_group_bf16(v.u, gs, lo, hi, code);
+        }
+        if constexpr (!CP) {
+            reinterpret_cast<uint2*>(q.xq + (size_t)row * (K >> 1))[g] = make_uint2(lo, hi);
+            q.sfb[((size_t)(g >> 4) * M + row) * 16 + (g & 15)] = (unsigned char)code;
+        } else {
+            // the four scale bytes of a 64-k block are in four neighbouring lanes (K % 256 == 0: all four exist)
+            const unsigned quad = 0xfu << (tid & 28);
+            uint32_t w = (uint32_t)code << (8 * (g & 3));
+            w |= __shfl_xor_sync(quad, w, 1);
+            w |= __shfl_xor_sync(quad, w, 2);
+            const size_t at = (size_t)(g >> 4) * q.nblk * 2048 + (size_t)((g & 15) >> 2) * 512;
+            #pragma unroll 4
+            for (int d = 0; d < ndst; ++d) {
+                reinterpret_cast<uint2*>(q.xq + (size_t)dst_row(d) * (K >> 1))[g] = make_uint2(lo, hi);
+                if ((g & 3) == 0) *reinterpret_cast<uint32_t*>(q.sfb + dst_sf(d) + at) = w;
+            }
+        }
+    };
+    #pragma unroll
+    for (int k = 0; k < KEEP; ++k) if (tid + k * THREADS < groups) emit(tid + k * THREADS, keep[k]);
+    for (int g = tid + KEEP * THREADS; g < groups; g += THREADS) { Grp v; load(g, v); emit(g, v); }
 }
 
+template <bool CP>
+static int quant_launch(int f32, const void* x, int M, int K, const ActQuant& q, cudaStream_t s) {
+    if (M < 1) return B200_OK;
+    const bool wide = K > 2048;                         // 128 threads hold the 128 groups of 2048 columns
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(M); lc.blockDim = dim3(wide ? 256 : 128); lc.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at; lc.numAttrs = 1;
+    auto kern = f32 ? (wide ? k_quant_act<true, CP, 256> : k_quant_act<true, CP, 128>) : (wide ? k_quant_act<false, CP, 256> : k_quant_act<false, CP, 128>);
+    if (cudaLaunchKernelEx(&lc, kern, x, M, K, q) != cudaSuccess) return launch_failed("k_quant_act");
+    return check_launch("k_quant_act");
+}
+int quant_act_launch(int f32, const void* x, int M, int K, const ActQuant& q, cudaStream_t s) { return quant_launch<true>(f32, x, M, K, q, s); }
+
 // ---- host side ---------------------------------------------------------------------------------
-static int gx_accumulators(int NT);
 static size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
+// Scale blocks of a dense call: its jobs have at least 64 columns unless there is one job (gx_plan), so the padding to
+// 128-token blocks at most doubles the rows.
+static size_t dense_sf_rows(int M) { return 2 * (((size_t)M + 127) / 128 * 128) + 256; }
 size_t gemm_mxf4_ws_bytes(int M, int K) {
     if (M < 1 || K < 256) return 256;
     const size_t rows = ((size_t)M + 255) / 256 * 256;
-    return up256(rows * (size_t)(K / 2)) + up256(rows * (size_t)(K / 16)) + up256(rows * 4);
+    return up256(rows * (size_t)(K / 2)) + up256(dense_sf_rows(M) * (size_t)(K / 16)) + up256(rows * 4);
 }
 
 bool gemm_mxf4_shape_ok(int K) {
@@ -439,79 +497,42 @@ bool gemm_mxf4_shape_ok(int K) {
     return !(K & 255) && K >= 256 && K <= 16384 && scale_box(K, &b, &z) && tmap_available();
 }
 
-int quant_act_launch(int mode, const void* x, const void* x2, float limit, const int* src_row, const int* m_dev, int M,
-                     int rows_launch, int K, unsigned char* xq, unsigned char* sfb, size_t sfb_rows, float* gsx, cudaStream_t s) {
-    if (rows_launch < 1) return B200_OK;
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(rows_launch); lc.blockDim = dim3(256); lc.dynamicSmemBytes = 0; lc.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    lc.attrs = at; lc.numAttrs = 1;
-    cudaError_t e;
-    if (mode == 0) e = cudaLaunchKernelEx(&lc, k_quant_act<0>, x, x2, limit, src_row, m_dev, M, K, xq, sfb, sfb_rows, gsx);
-    else if (mode == 1) e = cudaLaunchKernelEx(&lc, k_quant_act<1>, x, x2, limit, src_row, m_dev, M, K, xq, sfb, sfb_rows, gsx);
-    else e = cudaLaunchKernelEx(&lc, k_quant_act<2>, x, x2, limit, src_row, m_dev, M, K, xq, sfb, sfb_rows, gsx);
-    if (e != cudaSuccess) return launch_failed("k_quant_act");
-    return check_launch("k_quant_act");
+// Ring depth and TMEM columns of a launch; false where not even three stages (or two scale slots) fit.
+constexpr size_t GX_STATIC = 6 * 1024;                  // upper bound of the kernel's static shared memory
+static bool gx_layout(GxParams& p, int TA, long items_per_cta, size_t* smem) {
+    const int optin = 227 * 1024, nst = p.K / 256;
+    const size_t room = (size_t)optin - GX_STATIC - 1024;
+    p.nblk = gx_blocks(p.NT);
+    p.a_slot = ((uint32_t)p.R * 128u + 1023u) & ~1023u;
+    const int slot = 16 * TA + 16 * p.nblk;
+    // a second set of accumulators when there is a next item to overlap with and the columns allow it
+    p.nbuf = items_per_cta > 1 && 2 * TA * p.NT + 3 * slot <= GX_TMEM_COLS ? 2 : 1;
+    p.nslot = (GX_TMEM_COLS - p.nbuf * TA * p.NT) / slot;
+    const size_t stage = (size_t)TA * p.a_slot + (size_t)p.NT * 128 + (size_t)TA * 2048 + (size_t)p.nblk * 2048;
+    const long steps = std::min<long>(items_per_cta * nst, GX_MAX_STAGES);
+    p.stages = (int)std::min<size_t>((size_t)steps, room / stage);
+    p.nslot = std::min(p.nslot, p.stages);                // more would ask about a stage's use before last, whose barrier has moved on
+    if ((p.nslot < 2 && p.stages > 1) || p.stages < 1 || (p.stages < 3 && p.stages < steps)) return false;
+    p.b_off = (uint32_t)p.stages * TA * p.a_slot;
+    p.ts_off = p.b_off + (uint32_t)p.stages * p.NT * 128u;
+    p.sf_off = p.ts_off + (uint32_t)p.stages * TA * 2048u;
+    // the MMA reads 16 KB from the start of a weight slot whatever R: keep that inside the allocation
+    *smem = std::max((size_t)p.stages * stage, (size_t)(p.stages * TA - 1) * p.a_slot + 16384) + 1024;
+    return *smem <= room + 1024;
 }
 
-// Shared memory and stage count of a launch; false if not even two stages fit.
-template <int NT>
-static int gx_launch_t(GxParams& p, const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& ms, int grid, cudaStream_t s) {
-    auto kern = k_gemm_mxf4<NT>;
-    static int attr_cache[64][2] = {};               // [device] = {optin, static bytes + 1}
+template <bool TABLE, int TA, bool DUAL, int NBLK>
+static int gx_launch_n(const GxParams& p, const GxMaps& maps, int grid, size_t smem, cudaStream_t s) {
+    auto kern = k_gemm_mxf4<TABLE, TA, DUAL, NBLK>;
     static bool ready[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return launch_failed("gemm_mxf4: cudaGetDevice");
-    if (dev < 0 || dev >= 64) dev = 0;
-    int* ac = attr_cache[dev];
-    if (!ac[1]) {
+    if (dev < 0 || dev >= 64 || !ready[dev]) {
         cudaFuncAttributes fa;
-        int oi = 0;
-        if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess ||
-            cudaDeviceGetAttribute(&oi, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return launch_failed("gemm_mxf4: attributes");
-        ac[0] = oi; ac[1] = (int)fa.sharedSizeBytes + 1;
-    }
-    const size_t static_smem = (size_t)ac[1] - 1;
-    const size_t room = (size_t)ac[0] - static_smem - 2048;        // 1 KB alignment slack + 1 KB system reserve
-    const int nst = p.K / 256;
-    p.sps = p.sc_swz ? 8 : nst;
-    const int slabs = p.T * (nst / p.sps);
-    p.nacc = gx_accumulators(NT);
-    if (p.T < 1 || p.T * p.nacc * NT > GX_COL_SF || p.T * nst > GX_MAX_STEPS || slabs > GX_MAX_SLABS) return B200_ENOTIMPL;
-    p.nslot = std::min(slabs, 3);
-    const int nsteps = p.T * nst;
-    p.a_slot = ((uint32_t)p.R * 128u + 1023u) & ~1023u;
-    // Ring depths: a step is in flight from the moment its loads are issued until its MMAs complete, and both
-    // the weights (HBM) and the activations (L2, but requested by every CTA at once) take a microsecond or
-    // more to arrive, so the shallower of the two rings bounds the step rate.  Take the split of the shared
-    // memory that makes the shallower ring as deep as possible (ties: the deeper weight ring).
-    const size_t b_slot = (size_t)NT * 128 + (size_t)NT * 16, slab_sz = (size_t)p.nslot * p.R * p.sc_box;
-    p.sa = 0; p.sb = 0;
-    for (int sb = std::min(nsteps, 16); sb >= 1; --sb) {
-        const size_t fx = slab_sz + (size_t)sb * b_slot;
-        if (fx + (size_t)p.a_slot + GX_A_BYTES > room) continue;
-        const int sa = (int)std::min<size_t>((room - fx - GX_A_BYTES) / p.a_slot + 1, (size_t)std::min(nsteps, 16));
-        if (std::min(sa, sb) > std::min(p.sa, p.sb) || (std::min(sa, sb) == std::min(p.sa, p.sb) && sa > p.sa)) { p.sa = sa; p.sb = sb; }
-    }
-    if (const char* e = getenv("B200_GX_RINGS")) {       // tuning aid: "sa,sb" replaces the choice above when it fits
-        int ua = 0, ub = 0;
-        if (sscanf(e, "%d,%d", &ua, &ub) == 2 && ua >= 1 && ub >= 1 && ub <= 16 && ua <= 16) {
-            ua = std::min(ua, nsteps); ub = std::min(ub, nsteps);
-            if (slab_sz + (size_t)ub * b_slot + (size_t)(ua - 1) * p.a_slot + GX_A_BYTES <= room) { p.sa = ua; p.sb = ub; }
-        }
-    }
-    if (p.sa < 1 || (std::min(p.sa, p.sb) < 2 && nsteps > 1)) return B200_ENOTIMPL;
-    p.ssf = std::min(p.sb, (GX_TMEM_COLS - GX_COL_SF) / (16 + 4 * std::max(NT / 32, 4)));
-    const size_t fixed = slab_sz + (size_t)p.sb * b_slot;
-    // the MMA reads 16 KB from the start of a weight slot whatever R: keep that inside the allocation for the last slot
-    size_t smem = (size_t)p.sa * p.a_slot + fixed + 1024;
-    if (smem < (size_t)(p.sa - 1) * p.a_slot + GX_A_BYTES + 1024) smem = (size_t)(p.sa - 1) * p.a_slot + GX_A_BYTES + 1024;
-    if (!ready[dev]) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(ac[0] - static_smem)) != cudaSuccess)
-            return launch_failed("gemm_mxf4: cudaFuncSetAttribute");
-        ready[dev] = true;
+        if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || fa.sharedSizeBytes > GX_STATIC ||
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - GX_STATIC)) != cudaSuccess)
+            return launch_failed("gemm_mxf4: attributes");
+        if (dev >= 0 && dev < 64) ready[dev] = true;
     }
     cudaLaunchConfig_t lc{};
     lc.gridDim = dim3(grid); lc.blockDim = dim3(GX_THREADS); lc.dynamicSmemBytes = smem; lc.stream = s;
@@ -519,50 +540,37 @@ static int gx_launch_t(GxParams& p, const CUtensorMap& mx, const CUtensorMap& mw
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = at; lc.numAttrs = 1;
-    if (cudaLaunchKernelEx(&lc, kern, p, mx, mw, ms) != cudaSuccess) return launch_failed("k_gemm_mxf4");
+    if (cudaLaunchKernelEx(&lc, kern, p, maps) != cudaSuccess) return launch_failed("k_gemm_mxf4");
     return check_launch("k_gemm_mxf4");
 }
 
-static int gx_launch(int NT, GxParams& p, const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& ms, int grid, cudaStream_t s) {
-    switch (NT) {
-        case 32: return gx_launch_t<32>(p, mx, mw, ms, grid, s);
-        case 64: return gx_launch_t<64>(p, mx, mw, ms, grid, s);
-        case 128: return gx_launch_t<128>(p, mx, mw, ms, grid, s);
-        default: return gx_launch_t<256>(p, mx, mw, ms, grid, s);
+template <bool TABLE, int TA, bool DUAL>
+static int gx_launch(const GxParams& p, const GxMaps& maps, int grid, size_t smem, cudaStream_t s) {
+    return p.nblk == 1 ? gx_launch_n<TABLE, TA, DUAL, 1>(p, maps, grid, smem, s) : gx_launch_n<TABLE, TA, DUAL, 2>(p, maps, grid, smem, s);
+}
+
+// Shape of a dense call's items: (R, TA, NT) with the least estimated time.  An SM takes in about 115 B per ns and its
+// tensor pipe needs NT/2 clocks per 128 x NT x 64; a wave of items costs its steps at the slower of the two, plus its
+// epilogue where no second accumulator set hides it (5 ns per column and tile).  So few tokens get weight tiles just
+// low enough to give every SM one, and many get two 128-row tiles against a chunk of tokens that fills whole waves:
+// 512 tokens x 12288 rows run as 144 items of 256 rows x 176 tokens in one wave.
+static void gx_plan(int M, int N, int K, int nsm, int* R, int* TA, int* NT) {
+    const int nst = K / 256;
+    double best = -1.0;
+    for (int j = (M + GX_MAX_NT - 1) / GX_MAX_NT, k = 0; k < 8; ++k, ++j) {
+        const int nt = std::max(16, ((M + j - 1) / j + 15) & ~15), jobs = (M + nt - 1) / nt;
+        if (nt < 64 && jobs > 1) break;
+        for (int ta = 1; ta <= 2; ++ta) {
+            if (ta * nt + 2 * (16 * ta + 16 * gx_blocks(nt)) > GX_TMEM_COLS) continue;
+            for (int r = 16; r <= 128; r += 8) {
+                const long items = (long)((N + ta * r - 1) / (ta * r)) * jobs, waves = (items + nsm - 1) / nsm;
+                const double in = (ta * r * 144.0 + nt * 128.0 + gx_blocks(nt) * 2048.0) / 115.0, mma = ta * 4 * std::max(nt, 64) * 0.27;
+                const double epi = waves > 1 && 2 * ta * nt + 3 * (16 * ta + 16 * gx_blocks(nt)) <= GX_TMEM_COLS ? 1.0 : (double)waves;
+                const double t = waves * nst * std::max(in, mma) + epi * (ta * nt * 5.0 + 300.0);
+                if (best < 0.0 || t < best * 0.999) { best = t; *R = r; *TA = ta; *NT = nt; }
+            }
+        }
     }
-}
-
-// Token tile for M activation rows against N weight rows: as narrow as covers M up to 128; beyond
-// that 256 columns per CTA unless the narrower tile still fits one wave of CTAs.
-static int pick_nt(int M, int N) {
-    if (M <= 32) return 32;
-    if (M <= 64) return 64;
-    if (M <= 128) return 128;
-    const int tiles_n = (N + 127) / 128, nsm = sm_count();
-    return tiles_n * ((M + 127) / 128) <= nsm ? 128 : 256;
-}
-
-// Accumulators per tile.  The kernel can split a tile's k-blocks over 2 or 4 accumulators issued by two
-// warps (independent MMA chains); measured on B200 that buys nothing -- the steps are paced by the arrival
-// of the weight tiles, not by the MMA chain -- and it costs TMEM columns that are better spent on more tiles
-// per CTA, so one accumulator per tile it is.  B200_GX_NACC=2|4 switches the split on for experiments.
-static int gx_accumulators(int NT) {
-    static const int forced = [] { const char* e = getenv("B200_GX_NACC"); return e ? atoi(e) : 1; }();
-    if ((forced == 2 || forced == 4) && forced * NT <= GX_COL_SF) return forced;
-    return 1;
-}
-
-// Consecutive weight-row tiles per CTA: as many as the accumulator columns (T * NT <= 256), the per-step
-// barriers (T * K/256 <= 64) and the scale slabs allow while the launch still has a CTA for every SM.  A
-// CTA pays its set-up (TMEM, barriers, descriptors, pipeline fill and drain) once for all its tiles.
-static int pick_tiles_per_cta(int NT, int K, int tiles_n, long jobs) {
-    int box = 0, swz = 0;
-    scale_box(K, &box, &swz);
-    const int nst = K / 256, slabs_per_tile = swz ? nst / 8 : 1, nsm = sm_count();
-    int best = 1;
-    for (int T = 2; T <= tiles_n && T * gx_accumulators(NT) * NT <= GX_COL_SF && T * nst <= GX_MAX_STEPS && T * slabs_per_tile <= GX_MAX_SLABS; ++T)
-        if (jobs * ((tiles_n + T - 1) / T) >= nsm) best = T;
-    return best;
 }
 
 // Dense: y[M, N] = quant(x)[M, K] . W^T.  x_kind 0: bf16, 1: f32.  ws: gemm_mxf4_ws_bytes(M, K).
@@ -570,56 +578,54 @@ int gemm_mxf4_dense(float* y, const b200_wref* W, const void* x, int x_kind, int
     if (!y || !W || !W->packed || !W->scale || !W->gscale || !x || !ws || M < 1 || N < 1) return B200_EINVAL;
     if (!gemm_mxf4_shape_ok(K)) return B200_ENOTIMPL;
     if (((uintptr_t)W->packed & 15) || ((uintptr_t)W->scale & 15) || ((uintptr_t)x & 15) || ((uintptr_t)ws & 255)) return B200_ENOTIMPL;
-    const int NT = pick_nt(M, N), n_jobs = (M + NT - 1) / NT, nsm = sm_count();
-    // weight rows per CTA: with one token tile the kernel is bandwidth-bound and wants every SM busy (the
-    // smallest multiple of 8 whose tiles still fit the SMs); with several, the MMA is always 128 rows tall.
-    int R = 128;
-    if (n_jobs == 1)
-        for (int r = 8; r <= 128; r += 8) if ((N + r - 1) / r <= nsm) { R = r; break; }
+    const int nsm = sm_count();
+    GxParams p{};
+    int TA = 1;
+    gx_plan(M, N, K, nsm, &p.R, &TA, &p.NT);
+    p.K = K;
+    p.n_jobs = (M + p.NT - 1) / p.NT;
+    p.tiles = (N + TA * p.R - 1) / (TA * p.R);
+    const long items = (long)p.tiles * p.n_jobs;
+    const int grid = (int)std::min<long>(items, nsm);
+    size_t smem = 0;
+    if (!gx_layout(p, TA, (items + grid - 1) / grid, &smem)) return B200_ENOTIMPL;
     const size_t rows = ((size_t)M + 255) / 256 * 256;
     unsigned char* xq = static_cast<unsigned char*>(ws);
     unsigned char* sfb = xq + up256(rows * (size_t)(K / 2));
-    float* gsx = reinterpret_cast<float*>(sfb + up256(rows * (size_t)(K / 16)));
-    GxParams p{};
-    p.table = nullptr;
-    p.one = GxJob{y, W->gscale, gsx, nullptr, nullptr, 0, M, N, N};
-    p.sfb = sfb; p.sfb_rows = rows;
+    float* gsx = reinterpret_cast<float*>(sfb + up256(dense_sf_rows(M) * (size_t)(K / 16)));
+    p.one = GxJob{y, W->gscale, nullptr, gsx, nullptr, nullptr, W->scale, nullptr, sfb, 0, M, N, N};
     p.status = device_status_ptr();
     if (!p.status) return B200_ENOTIMPL;
-    p.n_jobs = n_jobs; p.K = K; p.R = R; p.prefetch_before_wait = stable_weights_option();
-    if (!scale_box(K, &p.sc_box, &p.sc_swz)) return B200_ENOTIMPL;
-    CUtensorMap mx, mw, ms;
-    if (!tmap_u8_2d(&mw, W->packed, (size_t)N, (size_t)K / 2, 128, R, true, true) ||
-        !tmap_u8_2d(&ms, W->scale, (size_t)N, (size_t)K / 16, p.sc_box, R, p.sc_swz != 0, true) ||
-        !tmap_u8_2d(&mx, xq, (size_t)M, (size_t)K / 2, 128, NT, true, true)) return B200_ENOTIMPL;
-    credit(B200_CREDIT_GEMM, (double)n_jobs * N * K * 0.5625);      // W streams once per token tile (the later tiles mostly from L2)
-    if (int rc = quant_act_launch(x_kind ? 1 : 0, x, nullptr, 0.f, nullptr, nullptr, M, n_jobs * NT, K, xq, sfb, rows, gsx, s)) return rc;
-    const int tiles_n = (N + R - 1) / R;
-    p.T = pick_tiles_per_cta(NT, K, tiles_n, n_jobs);
-    return gx_launch(NT, p, mx, mw, ms, (tiles_n + p.T - 1) / p.T * n_jobs, s);
+    p.prefetch_before_wait = stable_weights_option();
+    GxMaps maps;
+    if (!tmap_u8_2d(&maps.w, W->packed, (size_t)N, (size_t)K / 2, 128, p.R, true, true) ||
+        !tmap_u8_2d(&maps.x[0], xq, (size_t)M, (size_t)K / 2, 128, p.NT, true, true)) return B200_ENOTIMPL;
+    maps.x[1] = maps.x[2] = maps.x[3] = maps.x[0];
+    credit(B200_CREDIT_GEMM, (double)p.n_jobs * N * K * 0.5625);      // W streams once per token chunk (the later chunks mostly from L2)
+    const ActQuant q{xq, sfb, gsx, nullptr, nullptr, 1, p.NT, p.nblk};
+    if (int rc = quant_act_launch(x_kind, x, M, K, q, s)) return rc;
+    return TA == 2 ? gx_launch<false, 2, false>(p, maps, grid, smem, s) : gx_launch<false, 1, false>(p, maps, grid, smem, s);
 }
 
-// Jobs from a table in device memory (rows grouped by expert); expected_jobs: how many of the max_jobs slots
-// are likely to hold a job (decides how many tiles a CTA takes).  Every job's weight maps were encoded
-// with box height R and N weight rows; the activation rows of all jobs live in one quantised buffer
-// (xq [x_rows, K/2], scales sfb [K/256][sfb_rows][16]).
-int gemm_mxf4_table(const GxJob* table, int max_jobs, long expected_jobs, int NT, int N, int K, int R, const unsigned char* xq, size_t x_rows,
-                    const unsigned char* sfb, size_t sfb_rows, cudaStream_t s) {
+// Jobs from a table in device memory (rows grouped by expert), each of up to NT rows against matrices of N rows whose
+// maps were encoded with boxes 128 rows tall; the rows of all jobs lie in one quantised buffer xq [x_rows, K/2].
+int gemm_mxf4_table(const GxJob* table, const int* n_jobs, int NT, int N, int K, bool dual, float limit, const unsigned char* xq,
+                    size_t x_rows, cudaStream_t s) {
     if (!gemm_mxf4_shape_ok(K)) return B200_ENOTIMPL;
     GxParams p{};
-    p.table = table;
-    p.sfb = sfb; p.sfb_rows = sfb_rows;
+    p.table = table; p.n_jobs_dev = n_jobs; p.limit = limit;
     p.status = device_status_ptr();
     if (!p.status) return B200_ENOTIMPL;
-    p.n_jobs = max_jobs; p.K = K; p.R = R; p.prefetch_before_wait = 0;
-    if (!scale_box(K, &p.sc_box, &p.sc_swz)) return B200_ENOTIMPL;
-    CUtensorMap mx, mx32, mx64;                      // activation boxes of NT, 32 and 64 rows (jobs with few rows take the small ones)
-    if (!tmap_u8_2d(&mx, xq, x_rows, (size_t)K / 2, 128, NT, true, true) ||
-        !tmap_u8_2d(&mx32, xq, x_rows, (size_t)K / 2, 128, 32, true, true) ||
-        !tmap_u8_2d(&mx64, xq, x_rows, (size_t)K / 2, 128, 64, true, true)) return B200_ENOTIMPL;
-    const int tiles_n = (N + R - 1) / R;
-    p.T = pick_tiles_per_cta(NT, K, tiles_n, std::max(1L, expected_jobs));
-    return gx_launch(NT, p, mx, mx32, mx64, (tiles_n + p.T - 1) / p.T * max_jobs, s);
+    p.K = K; p.R = 128; p.NT = NT;
+    p.tiles = dual ? (N + 127) / 128 : (N + 255) / 256;
+    size_t smem = 0;
+    if (!gx_layout(p, 2, 1 << 20, &smem)) return B200_ENOTIMPL;
+    GxMaps maps;
+    const int box[4] = {NT, std::min(NT, 64), std::min(NT, 32), 16};
+    for (int k = 0; k < 4; ++k)
+        if (!tmap_u8_2d(&maps.x[k], xq, x_rows, (size_t)K / 2, 128, box[k], true, true)) return B200_ENOTIMPL;
+    maps.w = maps.x[0];
+    return dual ? gx_launch<true, 2, true>(p, maps, sm_count(), smem, s) : gx_launch<true, 2, false>(p, maps, sm_count(), smem, s);
 }
 
 }  // namespace b200
@@ -642,5 +648,6 @@ extern "C" int b200_nvfp4_quantize_tokens(const void* x, int x_is_f32, int M, in
     if (!x || !packed || !scale_step_major || !gs || M < 1 || K < 1) return B200_EINVAL;
     if (K & 255) return B200_ESHAPE;
     if (((uintptr_t)x & 15) || ((uintptr_t)packed & 7) || ((uintptr_t)scale_step_major & 15) || ((uintptr_t)gs & 3)) return B200_EALIGN;
-    return quant_act_launch(x_is_f32 ? 1 : 0, x, nullptr, 0.f, nullptr, nullptr, M, M, K, packed, scale_step_major, (size_t)M, gs, stream);
+    const ActQuant q{packed, scale_step_major, gs, nullptr, nullptr, 1, 0, 0};
+    return quant_launch<false>(x_is_f32 ? 1 : 0, x, M, K, q, stream);
 }

@@ -261,69 +261,89 @@ static int moe_umma_grouped(const float* x, const b200_moe_layer* L, float* y, c
 }
 
 // ---- 16 tokens and more: rows grouped by expert, both GEMM operands in NVFP4 -----------------------
-// Same counting sort as k_moe_group, but the jobs are those of the wide GEMM (gemm_mxf4.cu): one job
-// per expert and chunk of up to NT rows, so that an expert's weights are read once per NT rows that
-// chose it (the passes of 8 rows above re-read them NT/8 times).  src_row[pos] = token of the pair
-// sorted to position pos: the activation quantiser gathers with it.
+// Same counting sort as k_moe_group, but the jobs are those of the wide GEMM (gemm_mxf4.cu): one job per expert and
+// chunk of up to NT rows, so that an expert's weights are read once per NT rows that chose it (the passes of 8 rows
+// above re-read them NT/8 times).  pos[pair]: row of the pair in expert order; sfrow[pair], sfpos[row]: its column
+// among the activation scale blocks of the jobs (b200_internal.h, ActQuant).
+// Every CTA counts all pairs (64 KB of selections at 2048 tokens, from L2) and the ones before its own tokens, and
+// then places its own: no second launch and no waiting between CTAs.  One CTA for everything took 32 us at 2048
+// tokens, most of it in the scattered writes and the serial sum over the experts.
 __global__ void __launch_bounds__(1024)
-k_moe_group_gx(const __grid_constant__ MoePlan q, const int32_t* __restrict__ sel, int* __restrict__ posof,
-               int* __restrict__ src_row, GxJob* __restrict__ j1, GxJob* __restrict__ j2,
-               const float* __restrict__ gsx1, const float* __restrict__ gsx2, int M, int NT, int max_jobs,
+k_moe_group_gx(const __grid_constant__ MoePlan q, const int32_t* __restrict__ sel, int* __restrict__ pos,
+               int* __restrict__ sfrow, int* __restrict__ sfpos, GxJob* __restrict__ j1, GxJob* __restrict__ j2, int* __restrict__ n_jobs,
+               const unsigned char* __restrict__ sf1, const unsigned char* __restrict__ sf2,
+               const float* __restrict__ gsx1, const float* __restrict__ gsx2, int M, int NT, int tokens_per_cta,
                unsigned long long* __restrict__ credit_jobs) {
     __shared__ int cnt[MG_MAX_GROUPS], off[MG_MAX_GROUPS], jstart[MG_MAX_GROUPS], cursor[MG_MAX_GROUPS];
-    __shared__ int total_jobs;
+    pdl_launch_dependents();
     pdl_wait();
-    const int G = q.E + 1, pairs = M * q.ns;
-    for (int e = threadIdx.x; e < G; e += blockDim.x) { cnt[e] = 0; cursor[e] = 0; }
+    const int G = q.E + (q.ns > q.topk ? 1 : 0), tid = threadIdx.x;
+    const int m0 = blockIdx.x * tokens_per_cta, m1 = min(M, m0 + tokens_per_cta), npair = M * q.topk, before = m0 * q.topk;
+    for (int e = tid; e < G; e += blockDim.x) { cnt[e] = e < q.E ? 0 : M; cursor[e] = e < q.E ? 0 : m0; }
     __syncthreads();
-    auto group_of = [&](int p) {
-        const int m = p / q.ns, slot = p - m * q.ns;
-        if (slot >= q.topk) return q.E;
-        const int e = sel[(size_t)m * q.topk + slot];
-        return e < 0 ? 0 : (e >= q.E ? q.E - 1 : e);
-    };
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) atomicAdd(&cnt[group_of(p)], 1);
+    auto clamp_e = [&](int e) { return e < 0 ? 0 : (e >= q.E ? q.E - 1 : e); };
+    #pragma unroll 8
+    for (int p = tid; p < npair; p += 1024) {
+        const int e = clamp_e(sel[p]);
+        atomicAdd(&cnt[e], 1);
+        if (p < before) atomicAdd(&cursor[e], 1);
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (tid < 32) {                                      // exclusive sums of rows and of jobs over the experts
         int o = 0, j = 0;
-        for (int e = 0; e < G; ++e) { off[e] = o; jstart[e] = j; o += cnt[e]; j += (cnt[e] + NT - 1) / NT; }
-        total_jobs = j;
-        if (credit_jobs) { atomicAdd(&credit_jobs[0], 2ull * j); atomicAdd(&credit_jobs[1], (unsigned long long)j); }   // passes over expert matrices: gate + up, down
+        for (int e0 = 0; e0 < G; e0 += 32) {
+            const int e = e0 + tid, c = e < G ? cnt[e] : 0, cj = (c + NT - 1) / NT;
+            int so = c, sj = cj;
+            #pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int a = __shfl_up_sync(0xffffffffu, so, d), b = __shfl_up_sync(0xffffffffu, sj, d);
+                if (tid >= d) { so += a; sj += b; }
+            }
+            if (e < G) { off[e] = o + so - c; jstart[e] = j + sj - cj; }
+            o += __shfl_sync(0xffffffffu, so, 31); j += __shfl_sync(0xffffffffu, sj, 31);
+        }
+        if (tid == 0 && blockIdx.x == 0) {
+            *n_jobs = j;
+            if (credit_jobs) { atomicAdd(&credit_jobs[0], 2ull * j); atomicAdd(&credit_jobs[1], (unsigned long long)j); }   // passes over expert matrices: gate + up, down
+        }
     }
     __syncthreads();
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-        const int e = group_of(p), pos = off[e] + atomicAdd(&cursor[e], 1);
-        posof[p] = pos;
-        src_row[pos] = p / q.ns;
+    const int nblk = gx_blocks(NT), width = nblk * 128;
+    for (int k = tid; k < (m1 - m0) * q.ns; k += 1024) {
+        const int m = m0 + k / q.ns, slot = k % q.ns, e = slot < q.topk ? clamp_e(sel[(size_t)m * q.topk + slot]) : q.E;
+        const int rank = slot < q.topk ? atomicAdd(&cursor[e], 1) : m, row = off[e] + rank, c = rank / NT;
+        const int sr = (jstart[e] + c) * width + (rank - c * NT);
+        pos[m * q.ns + slot] = row;
+        sfrow[m * q.ns + slot] = sr;
+        sfpos[row] = sr;
     }
-    for (int e = threadIdx.x; e < G; e += blockDim.x) {
+    // the job records, dealt to the CTAs by expert
+    const size_t b1 = (size_t)(q.H >> 8) * nblk * 2048, b2 = (size_t)(q.I >> 8) * nblk * 2048;      // bytes of a job's scale blocks
+    for (int e = blockIdx.x + tid * gridDim.x; e < G; e += 1024 * gridDim.x) {
         const b200_nvfp4_mat* mats = e < q.E ? q.experts + (size_t)e * 3 : q.shared;
+        const b200_nvfp4_mat g = mats[0], u = mats[1], d = mats[2];
         const unsigned char* mp = q.maps + (size_t)(q.E + 1) * 6 * 128 + (size_t)e * 6 * 128;     // the 128-row boxes
         for (int c = 0; c * NT < cnt[e]; ++c) {
             const int idx = jstart[e] + c, rows = min(NT, cnt[e] - NT * c), pos0 = off[e] + NT * c;
-            j1[2 * idx] = GxJob{q.gbuf + (size_t)pos0 * q.I, mats[0].gscale, gsx1 + pos0, mp, mp + 128, pos0, rows, q.I, q.I};
-            j1[2 * idx + 1] = GxJob{q.ubuf + (size_t)pos0 * q.I, mats[1].gscale, gsx1 + pos0, mp + 256, mp + 384, pos0, rows, q.I, q.I};
-            j2[idx] = GxJob{q.part + (size_t)pos0 * q.H, mats[2].gscale, gsx2 + pos0, mp + 512, mp + 640, pos0, rows, q.H, q.H};
+            j1[idx] = GxJob{q.gbuf + (size_t)pos0 * q.I, g.gscale, u.gscale, gsx1 + pos0, mp, mp + 256, g.scale, u.scale, sf1 + idx * b1, pos0, rows, q.I, q.I};
+            j2[idx] = GxJob{q.part + (size_t)pos0 * q.H, d.gscale, nullptr, gsx2 + pos0, mp + 512, nullptr, d.scale, nullptr, sf2 + idx * b2, pos0, rows, q.H, q.H};
         }
-    }
-    for (int idx = total_jobs + threadIdx.x; idx < max_jobs; idx += blockDim.x) {
-        const GxJob none{nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 0};
-        j1[2 * idx] = none; j1[2 * idx + 1] = none; j2[idx] = none;
     }
 }
 
-// Token tile of the grouped wide GEMM: narrow while few rows share an expert (a job's cost is its
-// expert's weights whatever its width, and narrow tiles keep more stages in flight).
-static int gx_tile(int M) { return M <= 64 ? 32 : (M <= 256 ? 64 : 128); }
+// Token tile of the grouped wide GEMM: the most rows a job holds.  A job multiplies and loads only the rows it has, so a
+// wide tile costs ring depth and accumulator columns (64: two sets of accumulators), a narrow one re-reads the
+// weights of popular experts from L2.
+static int gx_tile(int M) { return M <= 512 ? 64 : 128; }
 static int gx_max_jobs(const b200_moe_layer* L, int M) { return (M * (L->topk + 1)) / gx_tile(M) + L->n_expert + 1; }
 
 static size_t moe_gx_ws_bytes(const b200_moe_layer* L, int M) {
-    const size_t np = (size_t)M * (L->topk + 1), mj = (size_t)gx_max_jobs(L, M), padrows = np + 256;
+    const size_t np = (size_t)M * (L->topk + 1), mj = (size_t)gx_max_jobs(L, M), sfrows = mj * gx_blocks(gx_tile(M)) * 128;
     const size_t H = L->hidden, I = L->inter;
-    return 2 * up256(np * 4) + up256(mj * 3 * sizeof(GxJob)) +
-           up256(np * (H / 2)) + up256(padrows * (H / 16)) + up256(np * 4) +          // quantised token rows
-           up256(np * (I / 2)) + up256(padrows * (I / 16)) + up256(np * 4) +          // quantised SwiGLU rows
-           2 * up256(np * I * 4) + up256(np * H * 4);                                 // gate, up, down products
+    return 3 * up256(np * 4) + 256 + up256(mj * 2 * sizeof(GxJob)) +
+           up256(np * (H / 2)) + up256(sfrows * (H / 16)) + up256(np * 4) +          // quantised token rows
+           up256(np * (I / 2)) + up256(sfrows * (I / 16)) + up256(np * 4) +          // quantised SwiGLU rows
+           up256(np * I * 4) + up256(np * H * 4);                                    // SwiGLU rows, down products
 }
 
 static int moe_gx_grouped(const float* x, const b200_moe_layer* L, float* y, const int32_t* sel, const float* wts,
@@ -333,35 +353,35 @@ static int moe_gx_grouped(const float* x, const b200_moe_layer* L, float* y, con
     if (!find_prepared(L, &Pc)) return B200_ENOTIMPL;
     const Prepared* P = &Pc;
     const int ns = L->topk + (L->shared ? 1 : 0), pairs = M * ns, H = L->hidden, I = L->inter;
-    const int NT = gx_tile(M), max_jobs = gx_max_jobs(L, M);
-    const size_t np = (size_t)M * (L->topk + 1), padrows = np + 256;
+    const int NT = gx_tile(M), max_jobs = gx_max_jobs(L, M), nblk = gx_blocks(NT);
+    const size_t np = (size_t)M * (L->topk + 1), sfrows = (size_t)max_jobs * nblk * 128;
     char* w = static_cast<char*>(scratch);
-    int* posof = reinterpret_cast<int*>(w); w += up256(np * 4);
-    int* src_row = reinterpret_cast<int*>(w); w += up256(np * 4);
-    GxJob* j1 = reinterpret_cast<GxJob*>(w); GxJob* j2 = j1 + (size_t)2 * max_jobs; w += up256((size_t)max_jobs * 3 * sizeof(GxJob));
+    int* pos = reinterpret_cast<int*>(w); w += up256(np * 4);
+    int* sfrow = reinterpret_cast<int*>(w); w += up256(np * 4);
+    int* sfpos = reinterpret_cast<int*>(w); w += up256(np * 4);
+    int* n_jobs = reinterpret_cast<int*>(w); w += 256;
+    GxJob* j1 = reinterpret_cast<GxJob*>(w); GxJob* j2 = j1 + max_jobs; w += up256((size_t)max_jobs * 2 * sizeof(GxJob));
     unsigned char* xq1 = reinterpret_cast<unsigned char*>(w); w += up256(np * (H / 2));
-    unsigned char* sf1 = reinterpret_cast<unsigned char*>(w); w += up256(padrows * (H / 16));
+    unsigned char* sf1 = reinterpret_cast<unsigned char*>(w); w += up256(sfrows * (H / 16));
     float* gs1 = reinterpret_cast<float*>(w); w += up256(np * 4);
     unsigned char* xq2 = reinterpret_cast<unsigned char*>(w); w += up256(np * (I / 2));
-    unsigned char* sf2 = reinterpret_cast<unsigned char*>(w); w += up256(padrows * (I / 16));
+    unsigned char* sf2 = reinterpret_cast<unsigned char*>(w); w += up256(sfrows * (I / 16));
     float* gs2 = reinterpret_cast<float*>(w); w += up256(np * 4);
     MoePlan q{};
-    q.gbuf = reinterpret_cast<float*>(w); w += up256(np * I * 4);
-    q.ubuf = reinterpret_cast<float*>(w); w += up256(np * I * 4);
+    q.gbuf = reinterpret_cast<float*>(w); w += up256(np * I * 4);      // SwiGLU rows
     q.part = reinterpret_cast<float*>(w);
     q.experts = L->experts; q.shared = L->shared; q.maps = P->maps; q.x = x;
     q.topk = L->topk; q.ns = ns; q.E = L->n_expert; q.H = H; q.I = I;
     if (credit_on()) credit_grouped_geometry(H, I);
-    k_moe_group_gx<<<1, 1024, 0, s>>>(q, sel, posof, src_row, j1, j2, gs1, gs2, M, NT, max_jobs, credit_on() ? credit_counters() : nullptr);
+    const int ctas = std::max(1, std::min(16, M / 64)), per = (M + ctas - 1) / ctas;
+    k_moe_group_gx<<<ctas, 1024, 0, s>>>(q, sel, pos, sfrow, sfpos, j1, j2, n_jobs, sf1, sf2, gs1, gs2, M, NT, per, credit_on() ? credit_counters() : nullptr);
     if (int rc = check_launch("k_moe_group_gx")) return rc;
-    if (int rc = quant_act_launch(1, x, nullptr, 0.f, src_row, nullptr, pairs, pairs, H, xq1, sf1, padrows, gs1, s)) return rc;
-    // jobs the table is likely to hold: every expert that can be hit once, plus the extra chunks of busy experts
-    const long expect = std::min<long>(L->n_expert, (long)M * L->topk) + (L->shared ? 1 : 0) + pairs / NT;
-    if (int rc = gemm_mxf4_table(j1, 2 * max_jobs, 2 * expect, NT, I, H, 128, xq1, (size_t)pairs, sf1, padrows, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
-    if (int rc = quant_act_launch(2, q.gbuf, q.ubuf, L->swiglu_limit, nullptr, nullptr, pairs, pairs, I, xq2, sf2, padrows, gs2, s)) return rc;
-    if (int rc = gemm_mxf4_table(j2, max_jobs, expect, NT, H, I, 128, xq2, (size_t)pairs, sf2, padrows, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
+    if (int rc = quant_act_launch(1, x, M, H, ActQuant{xq1, sf1, gs1, pos, sfrow, ns, NT, nblk}, s)) return rc;
+    if (int rc = gemm_mxf4_table(j1, n_jobs, NT, I, H, true, L->swiglu_limit, xq1, (size_t)pairs, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
+    if (int rc = quant_act_launch(1, q.gbuf, pairs, I, ActQuant{xq2, sf2, gs2, nullptr, sfpos, 1, NT, nblk}, s)) return rc;
+    if (int rc = gemm_mxf4_table(j2, n_jobs, NT, H, I, false, 0.f, xq2, (size_t)pairs, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
     const int y4 = M * (H >> 2);
-    k_moe_combine<<<(y4 + 255) / 256, 256, 0, s>>>(y, q.part, wts, posof, M, q.topk, ns, H);
+    k_moe_combine<<<(y4 + 255) / 256, 256, 0, s>>>(y, q.part, wts, pos, M, q.topk, ns, H);
     return check_launch("k_moe_combine");
 }
 

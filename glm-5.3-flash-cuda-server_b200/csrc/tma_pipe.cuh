@@ -75,6 +75,14 @@ __device__ __forceinline__ bool mbar_wait_spin(uint32_t bar, uint32_t parity, un
     atomicOr(status + 1, 1u << code);
     return false;
 }
+// One lane of a converged warp (always the same one).  Single-thread tcgen05 and TMA instructions belong behind this
+// and not behind `lane == 0`: their operands are warp-uniform registers, and only here does the compiler know that
+// one thread runs them.  Behind a lane test every such instruction took 40 to 80 ns to issue.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(ok));
+    return ok != 0;
+}
 // global -> shared bulk copy; dst, src 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
