@@ -90,32 +90,40 @@ k_gemm_f16w(const __grid_constant__ GfParams p, const __grid_constant__ CUtensor
     const uint32_t tmem = tmem_base_s;
 
     if (warp == 0) {
-        // ---- packed weights and their scales: lane l issues super-steps l, l + 32, .. ----
+        // ---- packed weights and their scales ----
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];" :: "l"(&map_w) : "memory");
             asm volatile("prefetch.tensormap [%0];" :: "l"(&map_s) : "memory");
         }
         if (!p.prefetch_before_wait) pdl_wait();
-        for (int g = lane; g < nsup; g += 32) {
+        for (int g = 0, sl = 0; g < nsup; ++g) {
             // the slot is free once the operand of the second half-step of the super-step that held it has been
             // converted (a16_full), not only multiplied: the MMAs never read the packed bytes
             if (g >= p.sp) mbar_wait_spin(smem_u32(&a16_full[2 * (g - p.sp) + 1]), 0, p.status, 21);
-            const uint32_t bar = smem_u32(&fullP[g]), dst = smem_u32(ringP) + (uint32_t)(g % p.sp) * GF_P_BYTES;
-            mbar_expect_tx(bar, GF_P_BYTES);
-            gf_tma_2d(dst, &map_w, g * 128, rown0, bar);
-            gf_tma_2d(dst + 16384, &map_s, g * 16, rown0, bar);                  // the super-step's 16 scale bytes of every row
+            if (elect_one()) {
+                const uint32_t bar = smem_u32(&fullP[g]), dst = smem_u32(ringP) + (uint32_t)sl * GF_P_BYTES;
+                mbar_expect_tx(bar, GF_P_BYTES);
+                gf_tma_2d(dst, &map_w, g * 128, rown0, bar);
+                gf_tma_2d(dst + 16384, &map_s, g * 16, rown0, bar);                  // the super-step's 16 scale bytes of every row
+            }
+            __syncwarp();
+            if (++sl == p.sp) sl = 0;
         }
         __syncwarp();
     } else if (warp == 3) {
-        // ---- activations: lane l issues half-steps l, l + 32, .. ----
+        // ---- activations ----
         if (lane == 0) asm volatile("prefetch.tensormap [%0];" :: "l"(&map_x) : "memory");
         pdl_wait();                                  // they come from the conversion launch
-        for (int h = lane; h < nhalf; h += 32) {
+        for (int h = 0, sl = 0; h < nhalf; ++h) {
             if (h >= p.sb) mbar_wait_spin(smem_u32(&done16[h - p.sb]), 0, p.status, 22);
-            const uint32_t bar = smem_u32(&fullB[h]), dst = smem_u32(ringB) + (uint32_t)(h % p.sb) * B_BYTES;
-            mbar_expect_tx(bar, B_BYTES);
-            gf_tma_2d(dst, &map_x, (2 * h) * 128, m0, bar);
-            gf_tma_2d(dst + NT * 128u, &map_x, (2 * h + 1) * 128, m0, bar);
+            if (elect_one()) {
+                const uint32_t bar = smem_u32(&fullB[h]), dst = smem_u32(ringB) + (uint32_t)sl * B_BYTES;
+                mbar_expect_tx(bar, B_BYTES);
+                gf_tma_2d(dst, &map_x, (2 * h) * 128, m0, bar);
+                gf_tma_2d(dst + NT * 128u, &map_x, (2 * h + 1) * 128, m0, bar);
+            }
+            __syncwarp();
+            if (++sl == p.sb) sl = 0;
         }
         __syncwarp();
         // asynchronous commit arrivals must have landed before the CTA's shared memory is handed on
@@ -129,7 +137,7 @@ k_gemm_f16w(const __grid_constant__ GfParams p, const __grid_constant__ CUtensor
             mbar_wait_spin(smem_u32(&a16_full[h]), 0, p.status, 24);
             mbar_wait_spin(smem_u32(&fullB[h]), 0, p.status, 25);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint64_t oA = (uint64_t)(((uint32_t)(h % p.na) * GF_A16_BYTES) >> 4), oB = (uint64_t)(((uint32_t)(h % p.sb) * B_BYTES) >> 4);
                 #pragma unroll
                 for (int kb = 0; kb < 2; ++kb) {
@@ -146,7 +154,7 @@ k_gemm_f16w(const __grid_constant__ GfParams p, const __grid_constant__ CUtensor
             }
             __syncwarp();
         }
-        if (lane == 0) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(&done_bar)) : "memory");
+        if (elect_one()) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(&done_bar)) : "memory");
         __syncwarp();
     } else if (warp >= 4 && warp < 12) {
         // ---- converters: thread -> (weight row r, k-block kb of the half-step) ----

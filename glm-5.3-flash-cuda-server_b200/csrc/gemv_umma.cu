@@ -22,8 +22,7 @@
 //   warp 0      TMA producer.  First the CTA's scale rows, as slabs [R rows x 128 B] (128B-swizzled,
 //               so 32 lanes reading one 16-byte column of 32 consecutive rows hit different banks);
 //               then per step one box [128 B x R rows] of packed weights (SWIZZLE_128B, the K-major
-//               operand layout the MMA reads) into a ring of stages.  Lane l issues steps l, l+32, ..:
-//               one thread issuing tensor loads back to back gets one out every ~0.35 us (measured).
+//               operand layout the MMA reads) into a ring of stages
 //   warp 1      L2 prefetch of the steps the ring cannot take at once; warps 2-3 idle
 //   warps 4-7   MMA issuers: warp w takes every fourth step: 4 tcgen05.mma (K = 64 each) into the
 //               accumulator of the step's k-block (k-block % 4: the summation order of a row never
@@ -41,8 +40,8 @@
 // parked at the closing barrier is scheduled rarely: measured 20 % slower).  Before it exits a CTA
 // waits for the last tcgen05.commit arrival of every stage: an arrival still in flight would land
 // in the shared memory of the next CTA on that SM.
-// Prologue without a CTA-wide barrier: warp 0 initialises the barriers of its own loads and requests the
-// slabs and the first four stages at once; the MMA warps initialise the other barriers, allocate TMEM and
+// Prologue without a CTA-wide barrier: warp 0 initialises the barriers of its own loads; the MMA warps
+// initialise the other barriers, allocate TMEM and
 // arrive at named barrier 3, where only the producer waits, and wait at named barrier 4, where the producer
 // arrives once its barriers are initialised; the workers go straight to the dependency wait and the
 // activation loads, and learn of everything else at named barrier 2.
@@ -98,7 +97,6 @@ struct UmParams {
     int sc_box, sc_swz;                            // scale slab: box width in bytes (128 swizzled, or K/16 plain)
     uint32_t bimg_off, scl_off, tsc_off;           // shared-memory offsets of the B image, of the scale slabs and (resident scales) of their transposed copy from the (1 KB aligned) ring
     int ov_first;                                  // resident scales: stages from this one on share their bytes with the scale slabs or the transposed copy
-    int early;                                     // stages requested by the producer before it waits for the other barriers (-1: not even the slabs)
     int acc_stride;                                // resident scales: TMEM columns between the four accumulators
     int require_res;                               // host only: refuse the launch unless it takes the resident-scales kernel
 };
@@ -298,12 +296,7 @@ k_gemv_umma(const __grid_constant__ UmParams p, const __grid_constant__ UmMaps m
     unsigned char* scl = ring + p.scl_off;          // all scale rows of the CTA: per tile, slabs [R x sc_box]
 
     pdl_launch_dependents();
-    // ---- TMA producer, part one (warp 0): with weights declared stable, the scale slabs and every stage that
-    // waits for nothing are requested before anything else happens in the CTA -- before the TMEM allocation and
-    // the CTA-wide barrier, on barriers this warp initialises itself.  Lane l issues steps l, l + 32, ...
     const uint32_t full0 = smem_u32(&full_bar[0]), ring0 = smem_u32(ring);
-    const int n_early = p.prefetch_before_wait ? min(min(p.stages, p.ov_first), p.early) : 0;
-    const bool early_scales = p.prefetch_before_wait && p.early >= 0;
     auto issue_scales = [&]() {
         // All scale rows of the CTA, in slabs [R rows x sc_box bytes]: one tensor load per slab instead of one
         // [R x 16 B] box per step (a box costs the TMA unit ~1 ns per row whatever the row's width).  128-byte
@@ -311,19 +304,27 @@ k_gemv_umma(const __grid_constant__ UmParams p, const __grid_constant__ UmMaps m
         // rows hit different banks.
         const int nslab = (K >> 4) / p.sc_box;
         const uint32_t slab_bytes = (uint32_t)p.R * (uint32_t)(K >> 4);     // one tile's scale rows
-        if (lane == 0) mbar_expect_tx(smem_u32(&sc_bar), slab_bytes * (uint32_t)T);
-        __syncwarp();
-        for (int q = lane; q < T * nslab; q += 32) {
-            const int t = q / nslab, sl = q - t * nslab;
-            tma_load_2d(smem_u32(scl) + (uint32_t)t * slab_bytes + (uint32_t)sl * (uint32_t)p.R * (uint32_t)p.sc_box,
-                        (const CUtensorMap*)J.ms, sl * p.sc_box, row0 + t * p.R, smem_u32(&sc_bar));
+        if (elect_one()) {
+            mbar_expect_tx(smem_u32(&sc_bar), slab_bytes * (uint32_t)T);
+            for (int t = 0; t < T; ++t)
+                for (int sl = 0; sl < nslab; ++sl)
+                    tma_load_2d(smem_u32(scl) + (uint32_t)t * slab_bytes + (uint32_t)sl * (uint32_t)p.R * (uint32_t)p.sc_box,
+                                (const CUtensorMap*)J.ms, sl * p.sc_box, row0 + t * p.R, smem_u32(&sc_bar));
         }
+        __syncwarp();
     };
-    auto issue_stage = [&](int g) {
-        const int s = g % p.stages, t = g / nst, it = g - t * nst;
-        const uint32_t bar = full0 + g * 8, dst = ring0 + (uint32_t)s * p.stage_bytes;
-        mbar_expect_tx(bar, (uint32_t)p.R * 128u);
-        tma_load_2d(dst, (const CUtensorMap*)J.mw, it * 128, row0 + t * p.R, bar);
+    // the producer's walk over the steps: next step, its stage, tile and k-block
+    int pg = 0, ps = 0, pt = 0, pit = 0;
+    auto issue_stage = [&]() {
+        if (elect_one()) {
+            const uint32_t bar = full0 + pg * 8;
+            mbar_expect_tx(bar, (uint32_t)p.R * 128u);
+            tma_load_2d(ring0 + (uint32_t)ps * p.stage_bytes, (const CUtensorMap*)J.mw, pit * 128, row0 + pt * p.R, bar);
+        }
+        __syncwarp();
+        ++pg;
+        if (++ps == p.stages) ps = 0;
+        if (++pit == nst) { pit = 0; ++pt; }
     };
     if (warp == 0) {
         for (int i = lane; i < nsteps; i += 32) mbar_init(full0 + i * 8, 1);
@@ -331,10 +332,6 @@ k_gemv_umma(const __grid_constant__ UmParams p, const __grid_constant__ UmMaps m
         mbar_fence_init();
         __syncwarp();
         asm volatile("bar.arrive 4, %0;" :: "r"(32 + 32 * UM_MMA_WARPS) : "memory");      // the MMA warps wait on these barriers before anyone else does
-        if (early_scales) {
-            issue_scales();
-            for (int g = lane; g < n_early; g += 32) issue_stage(g);
-        }
     }
     // No CTA-wide barrier in the prologue: the workers go straight to the dependency wait and the activation
     // loads (the longest chain of the kernel); the MMA warps initialise the other barriers and allocate TMEM,
@@ -389,22 +386,21 @@ k_gemv_umma(const __grid_constant__ UmParams p, const __grid_constant__ UmMaps m
     };
 
     if (warp < UM_LOAD_WARPS) {
-        // ---- TMA producer, part two: warp 0; lane l issues the loads of steps l, l + 32, ... ----
-        // One thread issuing tensor loads back to back gets one out every ~0.35 us (measured), so
-        // the steps are dealt to the lanes: each lane waits for its own stage and issues on its own.
+        // ---- TMA producer: the whole of warp 0 walks the steps and waits, one lane issues ----
         if (warp == 0) {
             const uint32_t empty0 = smem_u32(&empty_bar[0]);
-            if (!early_scales) {
-                if (lane == 0) { asm volatile("prefetch.tensormap [%0];" :: "l"(J.mw) : "memory");
-                                 asm volatile("prefetch.tensormap [%0];" :: "l"(J.ms) : "memory"); }
-                if (!p.prefetch_before_wait) pdl_wait();
-                issue_scales();
-            }
-            for (int g = lane; g < nsteps; g += 32) {
-                if (g < n_early) continue;
-                if (g >= p.stages) UM_WAIT(empty0 + (g - p.stages) * 8, 0, p.status, 1);      // the step that had this stage is done
-                else if (RES && g % p.stages >= p.ov_first) UM_WAIT(smem_u32(&scd_bar), 0, p.status, 8);   // the slabs under this stage are in TMEM
-                issue_stage(g);
+            // Nothing is requested before the MMA warps have met (about a microsecond into the CTA), not even with
+            // weights declared stable: requests from every SM at kernel entry delay what each needs first, its scale
+            // slabs and the activation row (six siblings, M = 1, us per launch: 7.6 so, 7.8 with the slabs at entry,
+            // 8.3 with four stages more, 8.6 with all 16; after the dependency wait 7.8, once the row is in 8.5).
+            if (lane == 0) { asm volatile("prefetch.tensormap [%0];" :: "l"(J.mw) : "memory");
+                             asm volatile("prefetch.tensormap [%0];" :: "l"(J.ms) : "memory"); }
+            if (!p.prefetch_before_wait) pdl_wait();
+            issue_scales();
+            while (pg < nsteps) {
+                if (pg >= p.stages) UM_WAIT(empty0 + (pg - p.stages) * 8, 0, p.status, 1);      // the step that had this stage is done
+                else if (RES && ps >= p.ov_first) UM_WAIT(smem_u32(&scd_bar), 0, p.status, 8);   // the slabs under this stage are in TMEM
+                issue_stage();
             }
             __syncwarp();
             // Tail: the tcgen05.commit arrivals on empty_bar are asynchronous.  Wait for the last one
@@ -459,7 +455,7 @@ k_gemv_umma(const __grid_constant__ UmParams p, const __grid_constant__ UmMaps m
             }
             fence_async_smem();
             __syncwarp();
-            if (lane == 0) {
+            if (elect_one()) {
                 for (int g = me; g < nsteps; g += UM_MMA_WARPS) {
                     #pragma unroll
                     for (int kb = 0; kb < 4; ++kb) {
@@ -501,7 +497,7 @@ k_gemv_umma(const __grid_constant__ UmParams p, const __grid_constant__ UmMaps m
         {
             int s = me % p.stages;
             int t = me / nst, it = me - t * nst;                       // tile and k-block of step g, kept without divisions
-            for (int g = me; g < nsteps; g += UM_MMA_WARPS) {          // whole warp waits, lane 0 issues
+            for (int g = me; g < nsteps; g += UM_MMA_WARPS) {          // whole warp waits, one lane issues
                 const uint32_t tsf = tmem + COL_SF + (uint32_t)(RES ? g : s) * 16u;
                 // accumulator it % 4 of tile t: fixed by the k-block alone, so that the summation order of a
                 // row does not depend on which tile of the CTA it is in (or on how many tiles a CTA takes)
@@ -511,7 +507,7 @@ k_gemv_umma(const __grid_constant__ UmParams p, const __grid_constant__ UmMaps m
                 UM_WAIT((RES ? full0 : sf0) + g * 8, 0, p.status, 3);      // resident scales: only the step's weights are awaited
                 if (!RES && g < npre) UM_WAIT(full0 + g * 8, 0, p.status, 2);   // scales moved ahead of the weights: wait for those too
                 tc_fence_after();
-                if (lane == 0) {
+                if (elect_one()) {
                     #pragma unroll
                     for (int kb = 0; kb < 4; ++kb) {                           // K % 256 == 0: always four 64-k blocks
                         asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
@@ -525,7 +521,7 @@ k_gemv_umma(const __grid_constant__ UmParams p, const __grid_constant__ UmMaps m
                 s += UM_MMA_WARPS; while (s >= p.stages) s -= p.stages;
                 it += UM_MMA_WARPS; while (it >= nst) { it -= nst; ++t; }
             }
-            if (lane == 0) tc_commit(smem_u32(&done_bar));
+            if (elect_one()) tc_commit(smem_u32(&done_bar));
             __syncwarp();
         }
     } else {
@@ -827,11 +823,6 @@ static int umma_finish_launch(UmParams& p, const UmMaps& maps, int tasks, cudaSt
     p.status = device_status_ptr();
     if (!p.status) return B200_ENOTIMPL;
     p.prefetch_before_wait = stable_weights_option();
-    // Measured on the decode shapes (six siblings, K = 4096, 16 stages resident): 4 stages at once 7.1-7.3 us per
-    // launch, 2: 7.5, 0: 7.7, 8: 7.9, all 16: 8.1-8.4.  A flood of requests from every SM at once delays what
-    // each SM needs first (its scale slabs, the activation row); pacing later requests by earlier arrivals was
-    // slower still (a window of 4 stages: 8.2, of 6: 7.5).
-    p.early = 4;
     if (p.dry_run) return B200_OK;
     const size_t smem = total + 1024;
     static bool ready_all[64][3] = {};               // the attribute is per device

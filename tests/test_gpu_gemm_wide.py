@@ -98,6 +98,28 @@ def test_gemm_bf16_vs_oracle(M, N, K):
     assert P.device_status() == 0
 
 
+# The persistent kernel's shapes: one and several items per CTA, one and two weight tiles per item (the second partly or
+# wholly out of range), one and two accumulator sets, 16 to 256 token columns, an odd number of 256-k steps
+@pytest.mark.parametrize('M,N,K', [(512, 3000, 1280), (512, 12200, 512), (1500, 2500, 512), (77, 5000, 1280), (200, 40000, 256), (130, 129, 768),
+                                   (240, 19000, 512)])
+def test_gemm_bf16_item_shapes_vs_dequantised_product(M, N, K):
+    """Against the same product in fp64 on the GPU (codes and weights are checked bit for bit elsewhere): only the
+    fp32 accumulation over K differs, K/64 roundings of 2^-24 each at most."""
+    P = pkg()
+    g = torch.Generator(device='cuda').manual_seed(M + N + K)
+    W = P.quantize((torch.randn((N, K), generator=g, device='cuda') * 0.02).to(torch.bfloat16))
+    x = torch.randn((M, K), generator=g, device='cuda').to(torch.bfloat16)
+    y = torch.full((M, N), float('nan'), device='cuda')
+    P.gemm_bf16(W, x, y)
+    p, sc, gs = P.quantize_tokens(x)
+    mag = torch.tensor([0, .5, 1, 1.5, 2, 3, 4, 6], device='cuda')
+    lut = torch.cat([mag, -mag])
+    v = torch.stack([lut[(p & 15).long()], lut[(p >> 4).long()]], -1).reshape(M, K) * sc.view(torch.float8_e4m3fn).float().repeat_interleave(16, 1)
+    ref = (v.double() / gs.double()[:, None]) @ P.dequantize(W).double().t()
+    assert ((y - ref).norm() / ref.norm()).item() <= K / 64 * 2.0 ** -24 + 1e-6      # + the fp32 rounding of dequantize()
+    assert P.device_status() == 0
+
+
 def test_gemm_bf16_token_independent_of_batch():
     """A token's row must not depend on the rest of the batch (its own global scale, its own MMA column)."""
     P = pkg()

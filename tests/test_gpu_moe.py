@@ -234,6 +234,13 @@ def test_moe_prefill_widths_run_the_grouped_wide_gemm(H, I, E, M, topk, shared, 
         P.moe_release(layer)
 
 
+@pytest.mark.parametrize('H,I,E,M,topk,shared', [(512, 768, 12, 600, 3, True), (768, 256, 5, 1100, 2, False), (256, 256, 40, 17, 2, True)])
+def test_moe_grouped_wide_gemm_job_shapes(H, I, E, M, topk, shared):
+    """Jobs of up to 128 rows and several chunks per expert, the grouping kernel on several CTAs, an odd number of 256-k
+    steps, one step only, jobs of one row; same checks as above."""
+    test_moe_prefill_widths_run_the_grouped_wide_gemm(H, I, E, M, topk, shared, True)
+
+
 def test_moe_prepared_layer_under_graph_capture():
     """The prepared path only launches kernels (descriptor look-up is host-side), so a layer forward
     can be captured and replayed; small-batch and grouped paths."""
