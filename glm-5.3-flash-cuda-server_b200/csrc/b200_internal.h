@@ -13,6 +13,18 @@ int sm_count();
 // cudaGetLastError() after a launch: 0, or B200_ELAUNCH with the runtime's text on stderr.
 int check_launch(const char* what);
 int launch_failed(const char* what);
+// Launch with programmatic stream serialisation: the kernel may start while its predecessor finishes and calls
+// pdl_wait() (tma_pipe.cuh) before it touches what that one wrote.
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = grid; lc.blockDim = block; lc.dynamicSmemBytes = smem; lc.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at; lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, kern, static_cast<P>(args)...);
+}
 // Device address of the status word that bounded waits write to (null if the query failed).
 unsigned int* device_status_ptr();
 // 1 if the caller declared weight buffers immutable while kernels run (B200_OPT_STABLE_WEIGHTS).

@@ -387,10 +387,22 @@ template <bool F32, bool CP, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 k_quant_act(const void* __restrict__ xin, int M, int K, const __grid_constant__ ActQuant q) {
     constexpr int KEEP = 2;
+    constexpr int MAX_DST = 20;                         // a token's slots: top-16 at most, and the shared expert
     __shared__ uint32_t red[THREADS / 32];
-    const int row = blockIdx.x, tid = threadIdx.x, groups = K >> 4;
+    __shared__ unsigned char* to_x[MAX_DST];            // where the row's codes and its column of scales go, per destination
+    __shared__ unsigned char* to_sf[MAX_DST];
+    const int row = blockIdx.x, tid = threadIdx.x, groups = K >> 4, nst = K >> 8, ndst = CP ? q.ndst : 1;
     pdl_launch_dependents();
     pdl_wait();
+    int drow = row;
+    if (CP && tid < ndst) {
+        if (q.pos) drow = q.pos[(size_t)row * ndst + tid];
+        int job, c;
+        if (q.sfrow) { const int s = q.sfrow[(size_t)row * ndst + tid], w = q.nblk * 128; job = s / w; c = s - job * w; }
+        else { job = row / q.NT; c = row - job * q.NT; }
+        to_x[tid] = q.xq + (size_t)drow * (K >> 1);
+        to_sf[tid] = q.sfb + ((size_t)job * nst * q.nblk + (c >> 7)) * 2048 + (size_t)((c & 31) * 16 + ((c & 127) >> 5) * 4);
+    }
     // eight words of a group: bf16 pairs as they lie in memory, or the sixteen floats
     struct Grp { uint32_t u[F32 ? 16 : 8]; };
     auto load = [&](int g, Grp& v) {
@@ -421,17 +433,7 @@ k_quant_act(const void* __restrict__ xin, int M, int K, const __grid_constant__ 
     #pragma unroll
     for (int w = 1; w < THREADS / 32; ++w) ai = max(ai, red[w]);
     const float gs = ai >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : nvfp4_global_scale(__uint_as_float(ai));
-    const int nst = K >> 8, ndst = CP ? q.ndst : 1;
-    // destination d of this row: packed row, and where its column of the scale blocks starts
-    auto dst_row = [&](int d) { return q.pos ? q.pos[(size_t)row * ndst + d] : row; };
-    auto dst_sf = [&](int d) -> size_t {
-        int job, c;
-        if (q.sfrow) { const int s = q.sfrow[(size_t)row * ndst + d], w = q.nblk * 128; job = s / w; c = s - job * w; }
-        else { job = row / q.NT; c = row - job * q.NT; }
-        return ((size_t)job * nst * q.nblk + (c >> 7)) * 2048 + (size_t)((c & 31) * 16 + ((c & 127) >> 5) * 4);
-    };
-    if (CP) { if (tid < ndst) q.gsx[dst_row(tid)] = gs; }
-    else if (tid == 0) q.gsx[row] = gs;
+    if (tid < ndst) q.gsx[drow] = gs;
     auto emit = [&](int g, const Grp& v) {
         uint32_t lo, hi; int code;
         if constexpr (F32) {
@@ -454,14 +456,69 @@ k_quant_act(const void* __restrict__ xin, int M, int K, const __grid_constant__ 
             const size_t at = (size_t)(g >> 4) * q.nblk * 2048 + (size_t)((g & 15) >> 2) * 512;
             #pragma unroll 4
             for (int d = 0; d < ndst; ++d) {
-                reinterpret_cast<uint2*>(q.xq + (size_t)dst_row(d) * (K >> 1))[g] = make_uint2(lo, hi);
-                if ((g & 3) == 0) *reinterpret_cast<uint32_t*>(q.sfb + dst_sf(d) + at) = w;
+                reinterpret_cast<uint2*>(to_x[d])[g] = make_uint2(lo, hi);
+                if ((g & 3) == 0) *reinterpret_cast<uint32_t*>(to_sf[d] + at) = w;
             }
         }
     };
     #pragma unroll
     for (int k = 0; k < KEEP; ++k) if (tid + k * THREADS < groups) emit(tid + k * THREADS, keep[k]);
     for (int g = tid + KEEP * THREADS; g < groups; g += THREADS) { Grp v; load(g, v); emit(g, v); }
+}
+
+// The same for f32 rows of up to GPL * 512 columns, one warp per row (the SwiGLU rows of a MoE layer: 18432 rows of 1536
+// columns at 2048 tokens).  The row stays in registers, the maximum is one warp reduction, and an SM holds 16 or 24
+// rows at different points of their load -> maximum -> codes chain; one CTA per row took 103 us there, its threads
+// idle for the most part (96 groups on 128 threads, a barrier, a double-precision quotient in the middle).
+template <int GPL>
+__global__ void __launch_bounds__(256, GPL <= 3 ? 3 : 2)
+k_quant_act_rows(const float* __restrict__ x, int M, int K, const __grid_constant__ ActQuant q) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, groups = K >> 4, nst = K >> 8;
+    if (row >= M) return;
+    float v[GPL][16];
+    const float4* r = reinterpret_cast<const float4*>(x + (size_t)row * K);
+    #pragma unroll
+    for (int k = 0; k < GPL; ++k)
+        if (lane + 32 * k < groups) {
+            #pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 a = r[(lane + 32 * k) * 4 + j];
+                v[k][4 * j] = a.x; v[k][4 * j + 1] = a.y; v[k][4 * j + 2] = a.z; v[k][4 * j + 3] = a.w;
+            }
+        }
+    uint32_t ai = 0u;
+    #pragma unroll
+    for (int k = 0; k < GPL; ++k)
+        if (lane + 32 * k < groups) {
+            #pragma unroll
+            for (int j = 0; j < 16; ++j) ai = max(ai, __float_as_uint(v[k][j]) & 0x7fffffffu);
+        }
+    ai = __reduce_max_sync(0xffffffffu, ai);
+    const float gs = ai >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : nvfp4_global_scale(__uint_as_float(ai));
+    for (int d = 0; d < q.ndst; ++d) {
+        const int to = q.pos ? q.pos[(size_t)row * q.ndst + d] : row;
+        int job, c;
+        if (q.sfrow) { const int s = q.sfrow[(size_t)row * q.ndst + d], w = q.nblk * 128; job = s / w; c = s - job * w; }
+        else { job = row / q.NT; c = row - job * q.NT; }
+        unsigned char* sf = q.sfb + ((size_t)job * nst * q.nblk + (c >> 7)) * 2048 + (size_t)((c & 31) * 16 + ((c & 127) >> 5) * 4);
+        if (lane == 0) q.gsx[to] = gs;
+        #pragma unroll
+        for (int k = 0; k < GPL; ++k) {
+            const int g = lane + 32 * k;
+            if (g < groups) {
+                uint32_t lo, hi; int code;
+                quantize_group(v[k], gs, lo, hi, code);
+                const unsigned quad = 0xfu << (lane & 28);
+                uint32_t w = (uint32_t)code << (8 * (g & 3));
+                w |= __shfl_xor_sync(quad, w, 1);
+                w |= __shfl_xor_sync(quad, w, 2);
+                reinterpret_cast<uint2*>(q.xq + (size_t)to * (K >> 1))[g] = make_uint2(lo, hi);
+                if ((g & 3) == 0) *reinterpret_cast<uint32_t*>(sf + (size_t)(g >> 4) * q.nblk * 2048 + (size_t)((g & 15) >> 2) * 512) = w;
+            }
+        }
+    }
 }
 
 template <bool CP>
@@ -478,7 +535,19 @@ static int quant_launch(int f32, const void* x, int M, int K, const ActQuant& q,
     if (cudaLaunchKernelEx(&lc, kern, x, M, K, q) != cudaSuccess) return launch_failed("k_quant_act");
     return check_launch("k_quant_act");
 }
-int quant_act_launch(int f32, const void* x, int M, int K, const ActQuant& q, cudaStream_t s) { return quant_launch<true>(f32, x, M, K, q, s); }
+int quant_act_launch(int f32, const void* x, int M, int K, const ActQuant& q, cudaStream_t s) {
+    // a warp per row where the rows alone fill the SMs (fewer rows are faster with a CTA each) and fit the registers
+    if (!f32 || K > 2048 || q.ndst != 1 || M < 16 * sm_count()) return quant_launch<true>(f32, x, M, K, q, s);
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3((M + 7) / 8); lc.blockDim = dim3(256); lc.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at; lc.numAttrs = 1;
+    auto kern = K <= 512 ? k_quant_act_rows<1> : K <= 1024 ? k_quant_act_rows<2> : K <= 1536 ? k_quant_act_rows<3> : k_quant_act_rows<4>;
+    if (cudaLaunchKernelEx(&lc, kern, static_cast<const float*>(x), M, K, q) != cudaSuccess) return launch_failed("k_quant_act_rows");
+    return check_launch("k_quant_act_rows");
+}
 
 // ---- host side ---------------------------------------------------------------------------------
 static size_t up256(size_t v) { return (v + 255) / 256 * 256; }

@@ -212,65 +212,78 @@ k_gemm_dense_row(float* __restrict__ y, const __nv_bfloat16* __restrict__ W, con
 }
 
 // The same product for MANY activation rows in one launch (the router logits of a prefill chunk): a CTA
-// takes ET weight rows x up to 8 activation rows.  Every (weight row, activation row) pair is computed
+// takes ET weight rows x TM activation rows.  Every (weight row, activation row) pair is computed
 // exactly as k_gemm_dense_row computes it -- same split of K over the threads, same FMA order, same
 // reduction order -- so a token's logits, and with them its expert selection, do not depend on how many
-// tokens were routed together.  Each thread keeps its slice of the 8 activation rows in registers and
-// reuses it for the ET weight rows.
-template <int ET>
-__global__ void __launch_bounds__(GEMV_THREADS)
-k_gemm_dense_rows(float* __restrict__ y, const __nv_bfloat16* __restrict__ W, const float* __restrict__ x, int M, int N, int K) {
-    constexpr int TM = 8;
-    __shared__ float part[GEMV_WARPS][ET][TM];
-    const int n0 = blockIdx.x * ET, m0 = blockIdx.y * TM, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int mv = min(TM, M - m0);
-    float acc[ET][TM];
+// tokens were routed together.  What bounds it is instruction issue: the FMAs of 2048 tokens x 144 experts x 4096 take
+// 33 us.  So a slice of an activation row, once in registers, meets ET weight rows, and the ET * TM partial sums of a
+// warp are reduced together: at each step of the butterfly a lane keeps half of the sums it has and sends the other
+// half, 2 (ET * TM / 32) + 31 shuffles at most instead of five for every sum.  A sum's tree of additions is the butterfly's.
+template <int N>                                   // N sums per lane -> the caller's lane keeps sums [first, first + N / 32) (N >= 32)
+__device__ __forceinline__ int warp_sum_many(float (&v)[N], int lane) {
+    int first = 0, n = N;
     #pragma unroll
-    for (int e = 0; e < ET; ++e)
+    for (int o = 16; o; o >>= 1) {
+        n >>= 1;
+        const bool up = lane & o;
         #pragma unroll
-        for (int m = 0; m < TM; ++m) acc[e][m] = 0.f;
-    for (int i = threadIdx.x; i < (K >> 3); i += GEMV_THREADS) {
-        float xr[TM][8];
-        #pragma unroll
-        for (int m = 0; m < TM; ++m) {
-            if (m < mv) {
-                const float4* xp = reinterpret_cast<const float4*>(x + (size_t)(m0 + m) * K + (size_t)i * 8);
-                const float4 a = xp[0], b = xp[1];
-                xr[m][0] = a.x; xr[m][1] = a.y; xr[m][2] = a.z; xr[m][3] = a.w; xr[m][4] = b.x; xr[m][5] = b.y; xr[m][6] = b.z; xr[m][7] = b.w;
-            } else {
-                #pragma unroll
-                for (int j = 0; j < 8; ++j) xr[m][j] = 0.f;
+        for (int k = 0; k < N / 2; ++k)
+            if (k < n) {
+                const float send = up ? v[k] : v[k + n], keep = up ? v[k + n] : v[k];
+                v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
             }
-        }
-        #pragma unroll
-        for (int e = 0; e < ET; ++e) {
-            if (n0 + e >= N) break;
-            const uint4 raw = reinterpret_cast<const uint4*>(W + (size_t)(n0 + e) * K)[i];
-            const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&raw);
-            float wf[8];
+        if (up) first += n;
+    }
+    return first;
+}
+template <int ET, int TM>
+__global__ void __launch_bounds__(GEMV_THREADS, 2)
+k_gemm_dense_rows(float* __restrict__ y, const __nv_bfloat16* __restrict__ W, const float* __restrict__ x, int M, int N, int K) {
+    constexpr int OUT = ET * TM;
+    __shared__ float part[GEMV_WARPS][OUT];
+    const int n0 = blockIdx.x * ET, m0 = blockIdx.y * TM, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float acc[OUT];                                  // sum of weight row e and activation row m at [e * TM + m]
+    #pragma unroll
+    for (int k = 0; k < OUT; ++k) acc[k] = 0.f;
+    // rows beyond the last one repeat it; their sums are not stored
+    const uint2* w0 = reinterpret_cast<const uint2*>(W + (size_t)n0 * K);
+    const float4* x0 = reinterpret_cast<const float4*>(x + (size_t)m0 * K);
+    const int ne = N - 1 - n0, nm = M - 1 - m0, k4 = K >> 2;
+    #pragma unroll 1
+    for (int i = threadIdx.x; i < (K >> 3); i += GEMV_THREADS) {
+        #pragma unroll 1
+        for (int h = 0; h < 2; ++h) {                // four of the eight elements at a time
+            uint2 raw[ET];
             #pragma unroll
-            for (int j = 0; j < 4; ++j) { const float2 f = __bfloat1622float2(b[j]); wf[2 * j] = f.x; wf[2 * j + 1] = f.y; }
+            for (int e = 0; e < ET; ++e) raw[e] = w0[min(e, ne) * k4 + 2 * i + h];
             #pragma unroll
-            for (int m = 0; m < TM; ++m) {
+            for (int mh = 0; mh < TM; mh += 4) {
+                float4 xv[4];
                 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[e][m] = fmaf(wf[j], xr[m][j], acc[e][m]);
+                for (int m = 0; m < 4; ++m) xv[m] = x0[min(mh + m, nm) * k4 + 2 * i + h];
+                #pragma unroll
+                for (int e = 0; e < ET; ++e) {
+                    const float wa = __uint_as_float(raw[e].x << 16), wb = __uint_as_float(raw[e].x & 0xffff0000u),
+                                wc = __uint_as_float(raw[e].y << 16), wd = __uint_as_float(raw[e].y & 0xffff0000u);
+                    #pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        float& c = acc[e * TM + mh + m];
+                        c = fmaf(wd, xv[m].w, fmaf(wc, xv[m].z, fmaf(wb, xv[m].y, fmaf(wa, xv[m].x, c))));
+                    }
+                }
             }
         }
     }
+    const int first = warp_sum_many<OUT>(acc, lane);
     #pragma unroll
-    for (int e = 0; e < ET; ++e)
-        #pragma unroll
-        for (int m = 0; m < TM; ++m) {
-            const float v = warp_sum(acc[e][m]);
-            if (lane == 0) part[warp][e][m] = v;
-        }
+    for (int k = 0; k < OUT / 32; ++k) part[warp][first + k] = acc[k];
     __syncthreads();
-    if (threadIdx.x < ET * TM) {
+    if (threadIdx.x < OUT) {
         const int e = threadIdx.x / TM, m = threadIdx.x - e * TM;
-        if (n0 + e < N && m < mv) {
+        if (n0 + e < N && m0 + m < M) {
             float v = 0.f;
             #pragma unroll
-            for (int w = 0; w < GEMV_WARPS; ++w) v += part[w][e][m];
+            for (int w = 0; w < GEMV_WARPS; ++w) v += part[w][threadIdx.x];
             y[(size_t)(m0 + m) * N + n0 + e] = v;
         }
     }
@@ -433,8 +446,12 @@ int dense_gemm(float* y, const void* W, const float* x, int M, int N, int K, int
     if (dtype != B200_F32 && dtype != B200_BF16) return B200_EINVAL;
     if (M > 8 && dtype == B200_BF16 && N <= 2048 && K >= 2048 && !(K & 7) && !((uintptr_t)W & 15) && !((uintptr_t)x & 15)) {
         // many rows against a small bf16 matrix (router logits of a prefill chunk): one launch, same bits per row
-        constexpr int ET = 4;
-        k_gemm_dense_rows<ET><<<dim3((N + ET - 1) / ET, (M + 7) / 8), GEMV_THREADS, 0, s>>>(y, static_cast<const __nv_bfloat16*>(W), x, M, N, K);
+        // 8 x 8 sums per thread once they fill the SMs twice over; below that smaller tiles and more CTAs
+        const __nv_bfloat16* w = static_cast<const __nv_bfloat16*>(W);
+        if ((long)((N + 7) / 8) * ((M + 7) / 8) >= 4L * sm_count())
+            k_gemm_dense_rows<8, 8><<<dim3((N + 7) / 8, (M + 7) / 8), GEMV_THREADS, 0, s>>>(y, w, x, M, N, K);
+        else
+            k_gemm_dense_rows<4, 8><<<dim3((N + 3) / 4, (M + 7) / 8), GEMV_THREADS, 0, s>>>(y, w, x, M, N, K);
         return check_launch("k_gemm_dense_rows");
     }
     for (int done = 0; done < M;) {

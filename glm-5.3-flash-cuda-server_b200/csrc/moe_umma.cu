@@ -83,27 +83,47 @@ __global__ void k_moe_plan(const __grid_constant__ MoePlan q, const int32_t* __r
 }
 
 // y[m, h] = sum over the routed slots in slot order of wts[m, k] * part[row(m, k), h], plus the shared expert's
-// row.  row(m, k) = m * ns + k, or posof[m * ns + k] when the rows were grouped by expert.
-__global__ void k_moe_combine(float* __restrict__ y, const float* __restrict__ part, const float* __restrict__ wts,
-                              const int* __restrict__ posof, int M, int topk, int ns, int H) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;          // float4 index
-    const int per = H >> 2;
-    if (i >= M * per) return;
-    const int m = i / per, h4 = i - m * per;
-    const float4* p = reinterpret_cast<const float4*>(part) + h4;
+// row.  row(m, k) = m * ns + k, or posof[m * ns + k] when the rows were grouped by expert.  Bound by HBM beyond a few
+// hundred tokens (302 MB of products at 2048): the rows' addresses are found first, so that a thread's loads are all
+// in flight before its first sum.
+constexpr int MC_MAX_SLOTS = 17;                      // topk <= 16, plus the shared expert
+__global__ void __launch_bounds__(256)
+k_moe_combine(float* __restrict__ y, const float* __restrict__ part, const float* __restrict__ wts,
+              const int* __restrict__ posof, int M, int topk, int ns, int H) {
+    __shared__ float w[MC_MAX_SLOTS];
+    __shared__ int row[MC_MAX_SLOTS];
+    const int m = blockIdx.y, per = H >> 2, i = blockIdx.x * 256 + threadIdx.x;      // float4 index within the token
+    if (threadIdx.x < ns) {
+        w[threadIdx.x] = threadIdx.x < topk ? wts[(size_t)m * topk + threadIdx.x] : 1.f;
+        row[threadIdx.x] = posof ? posof[m * ns + threadIdx.x] : m * ns + threadIdx.x;
+    }
+    __syncthreads();
+    if (i >= per) return;
+    const float4* p = reinterpret_cast<const float4*>(part) + i;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k = 0; k < topk; ++k) {
-        const float w = wts[(size_t)m * topk + k];
-        const int row = posof ? posof[m * ns + k] : m * ns + k;
-        const float4 v = p[(size_t)row * per];
-        acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y); acc.z = fmaf(w, v.z, acc.z); acc.w = fmaf(w, v.w, acc.w);
+    for (int k0 = 0; k0 < ns; k0 += 9) {
+        float4 v[9];
+        #pragma unroll
+        for (int k = 0; k < 9; ++k) if (k0 + k < ns) v[k] = p[(size_t)row[k0 + k] * per];
+        #pragma unroll
+        for (int k = 0; k < 9; ++k)
+            if (k0 + k < topk) {
+                const float f = w[k0 + k];
+                acc.x = fmaf(f, v[k].x, acc.x); acc.y = fmaf(f, v[k].y, acc.y); acc.z = fmaf(f, v[k].z, acc.z); acc.w = fmaf(f, v[k].w, acc.w);
+            } else if (k0 + k < ns) {
+                acc.x += v[k].x; acc.y += v[k].y; acc.z += v[k].z; acc.w += v[k].w;
+            }
     }
-    if (ns > topk) {
-        const int row = posof ? posof[m * ns + topk] : m * ns + topk;
-        const float4 v = p[(size_t)row * per];
-        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+    reinterpret_cast<float4*>(y)[(size_t)m * per + i] = acc;
+}
+static int combine_launch(float* y, const float* part, const float* wts, const int* posof, int M, int topk, int ns, int H, cudaStream_t s) {
+    for (int m0 = 0; m0 < M; m0 += 65535) {              // gridDim.y
+        const int c = std::min(M - m0, 65535);
+        const float* pt = posof ? part : part + (size_t)m0 * ns * H;
+        k_moe_combine<<<dim3(((H >> 2) + 255) / 256, c), 256, 0, s>>>(y + (size_t)m0 * H, pt, wts + (size_t)m0 * topk, posof ? posof + (size_t)m0 * ns : nullptr, c, topk, ns, H);
+        if (int rc = check_launch("k_moe_combine")) return rc;
     }
-    reinterpret_cast<float4*>(y)[i] = acc;
+    return B200_OK;
 }
 
 // ---- more than 8 tokens: rows grouped by expert ---------------------------------------------------
@@ -255,9 +275,7 @@ static int moe_umma_grouped(const float* x, const b200_moe_layer* L, float* y, c
     if (int rc = umma_table_launch(q.j1, 2 * max_jobs, I, H, P->R_gu, 0.f, 8, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
     if (int rc = umma_split_launch(s2, max_jobs, I, L->swiglu_limit, s)) return rc;
     if (int rc = umma_table_launch(q.j2, max_jobs, H, I, P->R_d, L->swiglu_limit, 8, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
-    const int y4 = M * (H >> 2);
-    k_moe_combine<<<(y4 + 255) / 256, 256, 0, s>>>(y, q.part, wts, posof, M, q.topk, ns, H);
-    return check_launch("k_moe_combine");
+    return combine_launch(y, q.part, wts, posof, M, q.topk, ns, H, s);
 }
 
 // ---- 16 tokens and more: rows grouped by expert, both GEMM operands in NVFP4 -----------------------
@@ -380,9 +398,7 @@ static int moe_gx_grouped(const float* x, const b200_moe_layer* L, float* y, con
     if (int rc = gemm_mxf4_table(j1, n_jobs, NT, I, H, true, L->swiglu_limit, xq1, (size_t)pairs, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
     if (int rc = quant_act_launch(1, q.gbuf, pairs, I, ActQuant{xq2, sf2, gs2, nullptr, sfpos, 1, NT, nblk}, s)) return rc;
     if (int rc = gemm_mxf4_table(j2, n_jobs, NT, H, I, false, 0.f, xq2, (size_t)pairs, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
-    const int y4 = M * (H >> 2);
-    k_moe_combine<<<(y4 + 255) / 256, 256, 0, s>>>(y, q.part, wts, pos, M, q.topk, ns, H);
-    return check_launch("k_moe_combine");
+    return combine_launch(y, q.part, wts, pos, M, q.topk, ns, H, s);
 }
 
 // The experts of a call on a prepared layer.  planned: the job tables were already written (by the router).
@@ -407,9 +423,7 @@ int moe_umma_experts(const float* x, const b200_moe_layer* L, float* y, const in
     }
     if (int rc = umma_table_launch(q.j1, 2 * pairs, q.I, q.H, R_gu, 0.f, 1, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
     if (int rc = umma_table_launch(q.j2, pairs, q.H, q.I, R_d, L->swiglu_limit, 1, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
-    const int n4 = M * (q.H >> 2);
-    k_moe_combine<<<(n4 + 255) / 256, 256, 0, s>>>(y, q.part, wts, nullptr, M, q.topk, q.ns, q.H);
-    return check_launch("k_moe_combine");
+    return combine_launch(y, q.part, wts, nullptr, M, q.topk, q.ns, q.H, s);
 }
 
 }  // namespace b200

@@ -14,14 +14,27 @@
 #include "b200_internal.h"
 #include "nvfp4_decode.cuh"
 #include "quant_core.cuh"
+#include "tma_pipe.cuh"
 
 namespace b200 {
 
+// gs = fp32(2688 / max(amax, 1e-12)), quotient in double, from the bits of amax.
+__device__ __forceinline__ float gs_of_bits(uint32_t bits) { return nvfp4_global_scale(__uint_as_float(bits)); }
+
+// The two words the maximum needs: its bits, and how many CTAs have added theirs (in the first bytes of the packed output,
+// which the code kernel overwrites; nullptr: not aligned).  It ends after everything before it in the stream has.
+__global__ void k_zero_words(uint32_t* a, uint32_t* b) {
+    pdl_wait();
+    *a = 0u;
+    if (b) *b = 0u;
+}
+
 // amax over the tensor.  Non-negative floats order like their bit patterns, so an unsigned
-// atomicMax on the bits is an exact, order-independent float max.
+// atomicMax on the bits is an exact, order-independent float max.  The last CTA turns the maximum into the scale.
 __global__ void __launch_bounds__(256)
 k_amax_bf16(const uint4* __restrict__ w, size_t n_vec, const __nv_bfloat16* __restrict__ tail,
-            size_t n_tail, uint32_t* __restrict__ out_bits) {
+            size_t n_tail, uint32_t* __restrict__ out_bits, uint32_t* __restrict__ done) {
+    pdl_launch_dependents();
     float a = 0.f;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -48,14 +61,23 @@ k_amax_bf16(const uint4* __restrict__ w, size_t n_vec, const __nv_bfloat16* __re
     if (blockIdx.x == 0)
         for (size_t i = threadIdx.x; i < n_tail; i += blockDim.x) a = fmaxf(a, fabsf(__bfloat162float(tail[i])));
     a = warp_max(a);
+    pdl_wait();                                      // the words are zero
     if ((threadIdx.x & 31) == 0 && a > 0.f) atomicMax(out_bits, __float_as_uint(a));
+    if (!done) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            *reinterpret_cast<float*>(out_bits) = gs_of_bits(atomicMax(out_bits, 0u));
+        }
+    }
 }
 
-// In place: amax bits -> gs = fp32(2688 / max(amax, 1e-12)), quotient in double.
+// In place: amax bits -> gs (an unaligned packed output, an empty tensor).
 __global__ void k_finish_gs(float* gs) {
-    double d = (double)gs[0];
-    if (!(d >= 1e-12)) d = 1e-12;
-    gs[0] = (float)((448.0 * 6.0) / d);
+    pdl_wait();
+    gs[0] = gs_of_bits(__float_as_uint(gs[0]));
 }
 
 __device__ __forceinline__ void unpack_bf16x16(const uint4& a, const uint4& b, float (&v)[16]) {
@@ -79,7 +101,8 @@ __device__ __forceinline__ void store_group(uint8_t* packed, uint8_t* scale, siz
 __global__ void __launch_bounds__(256)
 k_quantize(const __nv_bfloat16* __restrict__ w, size_t n_groups, const float* __restrict__ gsp,
            uint8_t* __restrict__ packed, uint8_t* __restrict__ scale, bool vec_in, bool vec_out) {
-    const float gs = gsp[0];
+    pdl_wait();
+    const float gs = *reinterpret_cast<const volatile float*>(gsp);
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (vec_in) {
@@ -146,24 +169,24 @@ extern "C" int b200_nvfp4_quantize(const void* w_bf16, int N, int K, uint8_t* pa
     const int grid_cap = sm_count() * 8;
     const float* gs = gscale_in;
     if (!gscale_in) {
-        if (cudaMemsetAsync(gscale, 0, 4, stream) != cudaSuccess) return launch_failed("quantize: memset");
+        uint32_t* bits = reinterpret_cast<uint32_t*>(gscale);
+        uint32_t* done = n && !((uintptr_t)packed & 3) ? reinterpret_cast<uint32_t*>(packed) : nullptr;
+        if (launch_pdl(k_zero_words, 1, 1, 0, stream, bits, done) != cudaSuccess) return launch_failed("k_zero_words");
         if (n) {
             const bool al = ((uintptr_t)w_bf16 & 15) == 0;
             const size_t n_vec = al ? n / 8 : 0, n_tail = n - n_vec * 8;
             const int grid = (int)std::min<size_t>((n_vec + 255) / 256 + 1, grid_cap);
-            k_amax_bf16<<<grid, 256, 0, stream>>>(static_cast<const uint4*>(w_bf16), n_vec,
-                static_cast<const __nv_bfloat16*>(w_bf16) + n_vec * 8, n_tail, reinterpret_cast<uint32_t*>(gscale));
-            if (int rc = check_launch("k_amax_bf16")) return rc;
+            if (launch_pdl(k_amax_bf16, grid, 256, 0, stream, static_cast<const uint4*>(w_bf16), n_vec,
+                           static_cast<const __nv_bfloat16*>(w_bf16) + n_vec * 8, n_tail, bits, done) != cudaSuccess) return launch_failed("k_amax_bf16");
         }
-        k_finish_gs<<<1, 1, 0, stream>>>(gscale);
-        if (int rc = check_launch("k_finish_gs")) return rc;
+        if (!done && launch_pdl(k_finish_gs, 1, 1, 0, stream, gscale) != cudaSuccess) return launch_failed("k_finish_gs");
         gs = gscale;
     }
     if (n == 0) return B200_OK;
     const size_t groups = n / 16;
     const int grid = (int)std::min<size_t>((groups + 255) / 256, grid_cap);
-    k_quantize<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(w_bf16), groups, gs, packed, scale,
-                                         ((uintptr_t)w_bf16 & 15) == 0, ((uintptr_t)packed & 7) == 0);
+    if (launch_pdl(k_quantize, grid, 256, 0, stream, static_cast<const __nv_bfloat16*>(w_bf16), groups, gs, packed, scale,
+                   ((uintptr_t)w_bf16 & 15) == 0, ((uintptr_t)packed & 7) == 0) != cudaSuccess) return launch_failed("k_quantize");
     return check_launch("k_quantize");
 }
 
