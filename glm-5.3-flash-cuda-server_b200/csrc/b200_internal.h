@@ -70,15 +70,13 @@ int nvfp4_multi_tma(const GemvParams& p, cudaStream_t s);
 int nvfp4_multi_umma(const GemvParams& p, int M, cudaStream_t s);
 size_t umma_presplit_bytes(int M, int K);
 int nvfp4_multi_umma_ws(const GemvParams& p, int M, void* ws, cudaStream_t s);
-// One job of the tensor-core kernel: x [M, K], y [M, N].  x2 != nullptr: the activations are the
-// clamped SwiGLU of two vectors, x = silu(min(x, limit)) * clamp(x2, -limit, limit) (the MoE down
-// projection reads the gate and up products directly).  mw, ms: CUtensorMap of packed weights and
+// One job of the tensor-core kernel: x [M, K], y [M, N].  mw, ms: CUtensorMap of packed weights and
 // of scales in GLOBAL memory (job-table launches); nullptr = the maps passed as kernel parameters.
 // bimg != nullptr: the activation rows were already split into their B image (K/256 x 8 KB, rows at a
-// stride of 8) and digit weights gam[M*8] by k_split_rows; x and x2 are then not read.
-struct UmJob { float* y; const float* x; const float* x2; const float* gs; const void* mw; const void* ms;
+// stride of 8) and digit weights gam[M*8] by k_split_rows; x is then not read.
+struct UmJob { float* y; const float* x; const float* gs; const void* mw; const void* ms;
                const unsigned char* bimg; const float* gam; int N; int M; int task0; int pad; };
-// One unit of k_split_rows: M rows of x (SwiGLU with x2 when x2 != nullptr) -> bimg, gam.  M = 0: nothing.
+// One unit of k_split_rows: M rows of x (when x2 != nullptr their clamped SwiGLU silu(min(x, limit)) * clamp(x2, -limit, limit)) -> bimg, gam.  M = 0: nothing.
 struct SplitJob { const float* x; const float* x2; unsigned char* bimg; float* gam; int M; int pad; };
 int umma_split_launch(const SplitJob* jobs, int n_jobs, int K, float limit, cudaStream_t s);
 bool umma_shape_ok(int K);
@@ -93,7 +91,7 @@ int moe_umma_experts(const float* x, const b200_moe_layer* L, float* y, const in
 int moe_experts_mode(const float* x, const b200_moe_layer* L, float* y, const int32_t* sel, const float* wts,
                      void* ws, int M, cudaStream_t s, int wide);
 int umma_encode_maps(void* out_w, void* out_s, const void* P, const void* S, int N, int K, int R);    // two 128-byte maps, host memory
-int umma_table_launch(const UmJob* table, int n_jobs, int N, int K, int R, float limit, int max_m, cudaStream_t s);
+int umma_table_launch(const UmJob* table, int n_jobs, int N, int K, int R, cudaStream_t s);
 
 // gemm_mxf4.cu: the wide GEMM with both operands in NVFP4 (activations quantised per token first).
 // One job: `rows` activation rows, starting at row `row0` of the quantised activation buffer, against one

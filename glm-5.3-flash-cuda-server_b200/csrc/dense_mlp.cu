@@ -4,11 +4,14 @@
 // (they share x), then the clamped SwiGLU, then down; from 16 rows on (and with the prefill option on)
 // the three products run on the wide tensor-core GEMM instead.
 #include "b200_internal.h"
+#include "tma_pipe.cuh"
 
 namespace b200 {
 
 __global__ void k_swiglu_clamped(float* __restrict__ out, const float* __restrict__ gate, const float* __restrict__ up,
                                  size_t n4, float limit) {
+    pdl_launch_dependents();                             // the down launch fetches its first weights meanwhile
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n4) return;
     const float4 a = reinterpret_cast<const float4*>(gate)[i], b = reinterpret_cast<const float4*>(up)[i];
@@ -48,7 +51,7 @@ extern "C" int b200_dense_mlp(const float* x, const b200_wref* gate, const b200_
         if (int rc = b200_nvfp4_gemm_ws(u, up, x, M, inter, hidden, B200_BF16, split, stream)) return rc;
     }
     const size_t n4 = (size_t)M * inter / 4;
-    k_swiglu_clamped<<<(unsigned)((n4 + 255) / 256), 256, 0, stream>>>(g, g, u, n4, limit);
+    if (launch_pdl(k_swiglu_clamped, (unsigned)((n4 + 255) / 256), 256, 0, stream, g, g, u, n4, limit) != cudaSuccess) return launch_failed("k_swiglu_clamped");
     if (int rc = check_launch("k_swiglu_clamped")) return rc;
     return b200_nvfp4_gemm_ws(y, down, g, M, hidden, inter, B200_BF16, split, stream);
 }

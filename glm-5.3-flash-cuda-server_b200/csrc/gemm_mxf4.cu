@@ -29,7 +29,7 @@
 // Every wait is bounded (tma_pipe.cuh).  No cluster launch, no multicast.
 #include "b200_internal.h"
 #include "quant_core.cuh"
-#include "tma_pipe.cuh"
+#include "umma_mxf4.cuh"
 #include <cuda.h>
 
 namespace b200 {
@@ -51,35 +51,6 @@ struct GxParams {
 };
 struct GxMaps { CUtensorMap w; CUtensorMap x[4]; };       // dense: weights; activations with boxes of NT rows (table: NT, 64, 32 and 16)
 
-__device__ __forceinline__ void gx_tma_2d(uint32_t dst, const void* map, int x, int y, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 :: "r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
-}
-__device__ __forceinline__ uint64_t gx_desc(uint32_t saddr) {
-    // K-major operand tile, 128B-swizzled: start address >> 4 | SBO = 1024 B (8 rows) | version 1 | SWIZZLE_128B
-    return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)(1024u >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-}
-__device__ __forceinline__ uint64_t gx_desc_sf(uint32_t saddr) {
-    // 32 rows x 16 B of scales, contiguous: four 8-row core matrices 128 B apart, no swizzle
-    return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | ((uint64_t)1 << 46);
-}
-__device__ __forceinline__ void gx_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void gx_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void gx_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
-}
-__device__ __forceinline__ void gx_cp_sf(uint32_t col, uint64_t desc) {
-    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" :: "r"(col), "l"(desc) : "memory");
-}
-__device__ __forceinline__ void gx_ld16(uint32_t col, float (&d)[16]) {
-    uint32_t v[16];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                 : "r"(col));
-    #pragma unroll
-    for (int j = 0; j < 16; ++j) d[j] = __uint_as_float(v[j]);
-}
 // The item's job and its weight-row tile.  A table's items go job by job (the tiles of an expert run side by side and
 // share its activation tile in L2), a dense call's tile by tile (the token chunks of a weight tile share the weights).
 struct GxItem { int job, tile; };
@@ -248,74 +219,18 @@ k_gemm_mxf4(const __grid_constant__ GxParams p, const __grid_constant__ GxMaps m
             }
         }
     } else if (warp >= 4 && warp < 8) {
-        // ---- weight scales.  A unit is two steps of one weight tile; warp w takes every NW-th unit. ----
-        // NW keeps a warp's consecutive units at most S steps apart: a warp sees only its own uses of a stage, and further
-        // apart it could ask for a phase of empty_bar whose predecessor has not completed either (a parity cannot tell).
-        const int NW = TA == 2 ? (S >= 4 ? 4 : 2) : max(1, min(4, S >> 1));
+        // ---- weight scales ----
         if (!TABLE && !p.prefetch_before_wait) pdl_wait();
-        const int pairs = (nst + 1) >> 1, upi = pairs * TA;
-        const size_t pitch = (size_t)(K >> 4);
-        const unsigned char* scp[TA];                  // of item ci: the tile's first scale row
-        int ci = -1, rows_t[TA];
-        auto load = [&](int i, int u, uint4 (&v)[2][4]) {
-            if (i != ci) {
-                ci = i;
-                const GxItem q = gx_item<TABLE>(p, first + i * stride);
-                #pragma unroll
-                for (int t = 0; t < TA; ++t) {
-                    const unsigned char* sc = TABLE ? (DUAL && t ? p.table[q.job].sc2 : p.table[q.job].sc) : p.one.sc;
-                    const int N = TABLE ? p.table[q.job].N : p.one.N, r0 = q.tile * nrow + (DUAL ? 0 : t * R);
-                    scp[t] = sc + (size_t)r0 * pitch;
-                    rows_t[t] = min(R, N - r0);
-                    // the tile's scale rows, asked into L2 by one warp
-                    if (warp == 4 + t)
-                        for (int r = lane; r < rows_t[t]; r += 32)
-                            for (size_t o = 0; o < pitch; o += 128)
-                                asm volatile("prefetch.global.L2 [%0];" :: "l"(scp[t] + (size_t)r * pitch + o));
-                }
+        move_weight_scales<TA>([&](int i, const unsigned char* (&sc)[TA], int (&rows)[TA]) {
+            const GxItem q = gx_item<TABLE>(p, first + i * stride);
+            const int N = TABLE ? p.table[q.job].N : p.one.N;
+            #pragma unroll
+            for (int t = 0; t < TA; ++t) {
+                const int r0 = q.tile * nrow + (DUAL ? 0 : t * R);
+                sc[t] = (TABLE ? (DUAL && t ? p.table[q.job].sc2 : p.table[q.job].sc) : p.one.sc) + (size_t)r0 * (size_t)(K >> 4);
+                rows[t] = min(R, N - r0);
             }
-            const int t = TA == 2 ? (u & 1) : 0, st = (TA == 2 ? u >> 1 : u) * 2;
-            const unsigned char* base = (TA == 2 && t ? scp[TA - 1] : scp[0]) + (size_t)st * 16;
-            const int rv = TA == 2 && t ? rows_t[TA - 1] : rows_t[0];
-            #pragma unroll
-            for (int h = 0; h < 2; ++h)
-                #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int r = lane + 32 * c;
-                    v[h][c] = (r < rv && st + h < nst) ? __ldg(reinterpret_cast<const uint4*>(base + (size_t)r * pitch + h * 16)) : make_uint4(0u, 0u, 0u, 0u);
-                }
-        };
-        int i = 0, u = warp - 4;
-        auto settle = [&] { while (u >= upi) { u -= upi; ++i; } };
-        uint4 v[2][4];
-        if (u >= NW) i = n_items;                       // an idle warp
-        settle();
-        if (i < n_items) load(i, u, v);
-        while (i < n_items) {
-            const int g0 = i * nst + (TA == 2 ? u >> 1 : u) * 2, t = TA == 2 ? (u & 1) : 0;
-            const int left = (i + 1) * nst - g0;       // steps of the item from this one on
-            uint4 cur[2][4];
-            #pragma unroll
-            for (int h = 0; h < 2; ++h)
-                #pragma unroll
-                for (int c = 0; c < 4; ++c) cur[h][c] = v[h][c];
-            u += NW; settle();
-            if (i < n_items) load(i, u, v);
-            #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                if (h >= left) break;
-                const int g = g0 + h, use = g / S, s = g - use * S;
-                mbar_wait_spin(empty0 + s * 8, (use & 1) ^ 1, p.status, 13);
-                uint4* o = reinterpret_cast<uint4*>(ringA + p.ts_off + (size_t)(s * TA + t) * 2048) + lane;
-                o[0] = make_uint4(cur[h][0].x, cur[h][1].x, cur[h][2].x, cur[h][3].x);
-                o[32] = make_uint4(cur[h][0].y, cur[h][1].y, cur[h][2].y, cur[h][3].y);
-                o[64] = make_uint4(cur[h][0].z, cur[h][1].z, cur[h][2].z, cur[h][3].z);
-                o[96] = make_uint4(cur[h][0].w, cur[h][1].w, cur[h][2].w, cur[h][3].w);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // generic-proxy stores -> the copy's async-proxy reads
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full0 + s * 8);
-            }
-        }
+        }, n_items, nst, S, ringA + p.ts_off, full0, empty0, p.status, warp - 4, lane);
     } else if (warp >= 8) {
         // ---- epilogue: two groups of four warps (one per TMEM lane quadrant) take alternate 16-token chunks ----
         const int te = tid - 256, grp = te >> 7, q4 = warp & 3, r = q4 * 32 + lane;

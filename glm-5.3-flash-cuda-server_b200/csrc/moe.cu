@@ -30,14 +30,19 @@ struct MoeArgs {
     float limit;
 };
 
-// One warp per token.  Ranking value = sigmoid(logit) + bias, gate value = sigmoid(logit);
+// One warp per token (and, where the experts run on moe_stream.cu, eight more that write the digits of its row meanwhile).
+// Ranking value = sigmoid(logit) + bias, gate value = sigmoid(logit);
 // among equal ranking values the lowest expert index wins, as in the reference's serial scan
 // with a strict '>' (kernels/moe.cu:146-152).
 template <int C>                                   // candidates per lane: n_expert <= 32 * C
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(UM_WORKERS + 32)
 k_route(int32_t* __restrict__ sel, float* __restrict__ wts, const float* __restrict__ logits,
         const float* __restrict__ bias, int E, int K, float scaling, int norm_prob, const __grid_constant__ MoePlan plan) {
-    const int tok = blockIdx.x, lane = threadIdx.x;
+    const int tok = blockIdx.x, lane = threadIdx.x & 31;
+    pdl_launch_dependents();
+    pdl_wait();
+    __shared__ float red[UM_MAX_M][8];
+    if (plan.maps && threadIdx.x < UM_WORKERS) { moe_plan_split(plan, tok, red, (int)threadIdx.x); return; }
     logits += (size_t)tok * E; sel += (size_t)tok * K; wts += (size_t)tok * K;
     // Ranking values as unsigned keys that order like the floats (0 = not a candidate: padding, a NaN, anything
     // at or below -1e30, or already taken), so that a round is two warp reductions -- the largest key, then the
@@ -86,7 +91,7 @@ k_route(int32_t* __restrict__ sel, float* __restrict__ wts, const float* __restr
     }
     if (lane < K) wts[lane] = my_w / d * scaling;
     // job records of the tensor-core experts for this token's pairs (prepared layers only)
-    if (plan.j1 && lane < plan.ns) moe_plan_pair(plan, tok, lane, my_e);
+    if (plan.maps && lane < plan.ns) moe_plan_pair(plan, tok, lane, my_e);
 }
 
 template <int MATH>
@@ -272,12 +277,9 @@ static int route_launch(const float* x, const b200_moe_layer* L, int32_t* sel, f
     if (int rc = check_layer(L, M)) return rc;
     if (!x || !sel || !wts || !logits || !L->router_bias) return B200_EINVAL;
     if (int rc = b200_nvfp4_gemm(logits, &L->router_w, x, M, L->n_expert, L->hidden, B200_BF16, stream)) return rc;
-    if (L->n_expert <= 128)
-        k_route<4><<<M, 32, 0, stream>>>(sel, wts, logits, L->router_bias, L->n_expert, L->topk, L->routed_scale, L->norm_topk, plan);
-    else if (L->n_expert <= 256)
-        k_route<8><<<M, 32, 0, stream>>>(sel, wts, logits, L->router_bias, L->n_expert, L->topk, L->routed_scale, L->norm_topk, plan);
-    else
-        k_route<ROUTE_MAXC><<<M, 32, 0, stream>>>(sel, wts, logits, L->router_bias, L->n_expert, L->topk, L->routed_scale, L->norm_topk, plan);
+    auto kern = L->n_expert <= 128 ? k_route<4> : L->n_expert <= 256 ? k_route<8> : k_route<ROUTE_MAXC>;
+    if (launch_pdl(kern, M, plan.maps ? UM_WORKERS + 32 : 32, 0, stream, sel, wts, static_cast<const float*>(logits), L->router_bias, L->n_expert, L->topk,
+                   L->routed_scale, L->norm_topk, plan) != cudaSuccess) return launch_failed("k_route");
     return check_launch("k_route");
 }
 

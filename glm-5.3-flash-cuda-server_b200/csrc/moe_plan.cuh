@@ -1,16 +1,24 @@
-// moe_plan.cuh -- job records of the tensor-core MoE path for one (token, slot) pair.
+// moe_plan.cuh -- job records and digit rows of the tensor-core MoE path for one (token, slot) pair.
 #pragma once
 #include "b200_internal.h"
+#include "digit_split.cuh"
 
 namespace b200 {
 
+// One activation row against one expert matrix, or its gate and its up matrix (moe_stream.cu).  img: the row's digits
+// [K/256][8 digits][128 B], gam: their weights.  mw, mw2: tensor maps of packed weights in GLOBAL memory; sc, sc2: their scales.
+struct MsJob { float* y; const float* gs; const float* gs2; const void* mw; const void* mw2; const unsigned char* sc;
+               const unsigned char* sc2; const unsigned char* img; const float* gam; };
+
 // Where the job tables, the per-expert tensor maps and the intermediate buffers of one call live.
-// j1 == nullptr: no plan wanted.
+// maps == nullptr: no plan wanted.
 struct MoePlan {
-    UmJob* j1; UmJob* j2;                          // gate/up jobs [2 * pairs], down jobs [pairs]
+    MsJob* j1; MsJob* j2;                          // gate and up, down: one job per pair each
     const b200_nvfp4_mat* experts; const b200_nvfp4_mat* shared;
     const unsigned char* maps;                     // [(E + 1) experts][gate w,s | up w,s | down w,s] x 128 bytes
     const float* x; float* gbuf; float* ubuf; float* part;
+    unsigned char* img1; unsigned char* img2;      // digits of the token rows and of the SwiGLU rows
+    float* gam1; float* gam2;
     int topk, ns, E, H, I;
 };
 
@@ -20,13 +28,20 @@ __device__ __forceinline__ void moe_plan_pair(const MoePlan& q, int m, int slot,
     const b200_nvfp4_mat* mats = q.shared;
     if (slot < q.topk) { e = e < 0 ? 0 : (e >= q.E ? q.E - 1 : e); mats = q.experts + (size_t)e * 3; }
     else e = q.E;                                  // the shared expert's maps come last
+    const b200_nvfp4_mat g = mats[0], u = mats[1], d = mats[2];
     const unsigned char* mp = q.maps + (size_t)e * 6 * 128;
-    const float* xm = q.x + (size_t)m * q.H;
-    float* g = q.gbuf + (size_t)pair * q.I;
-    float* u = q.ubuf + (size_t)pair * q.I;
-    q.j1[2 * pair] = UmJob{g, xm, nullptr, mats[0].gscale, mp, mp + 128, nullptr, nullptr, q.I, 1, 0, 0};
-    q.j1[2 * pair + 1] = UmJob{u, xm, nullptr, mats[1].gscale, mp + 256, mp + 384, nullptr, nullptr, q.I, 1, 0, 0};
-    q.j2[pair] = UmJob{q.part + (size_t)pair * q.H, g, u, mats[2].gscale, mp + 512, mp + 640, nullptr, nullptr, q.H, 1, 0, 0};
+    q.j1[pair] = MsJob{q.gbuf + (size_t)pair * q.I, g.gscale, u.gscale, mp, mp + 256, g.scale, u.scale,
+                       q.img1 + (size_t)m * q.H * 4, q.gam1 + m * UM_NB};
+    q.j2[pair] = MsJob{q.part + (size_t)pair * q.H, d.gscale, nullptr, mp + 512, nullptr, d.scale, nullptr,
+                       q.img2 + (size_t)pair * q.I * 4, q.gam2 + pair * UM_NB};
 }
+
+// Token m's row into digits, by UM_WORKERS threads (t = 0 .. UM_WORKERS - 1).
+__device__ __forceinline__ void moe_plan_split(const MoePlan& q, int m, float (*red)[8], int t) {
+    split_rows<true>(q.x + (size_t)m * q.H, nullptr, 0.f, 1, q.H, 1, q.img1 + (size_t)m * q.H * 4, q.gam1 + m * UM_NB, red, t);
+}
+
+int moe_stream_plan_launch(const MoePlan& q, const int32_t* sel, int M, cudaStream_t s);
+int moe_stream_launch(const MoePlan& q, int M, int R_gu, int R_d, float limit, cudaStream_t s);
 
 }  // namespace b200

@@ -28,6 +28,7 @@
 namespace b200 {
 
 constexpr int MU_MAX_TOKENS = 8;
+constexpr size_t MS_PAIR_BYTES = 2 * sizeof(MsJob) + 2 * UM_NB * sizeof(float);     // two job records, two rows of digit weights
 // Fewest tokens for which the (token, slot) pairs are sorted by expert, so that every distinct expert
 // (and the shared expert) is streamed once for up to 8 rows instead of once per pair (the reference's
 // gathered kernels, kernels/moe.cu:353-581).  Below it every pair is its own job.  B200_MOE_GROUP_MIN
@@ -63,23 +64,16 @@ static bool find_prepared(const b200_moe_layer* L, Prepared* out) {
     return false;
 }
 
-// Box height for n_jobs jobs of N rows: fewest waves of CTAs over the SMs, each wave costing its
-// rows plus a fixed part (activation split, pipeline fill and drain) worth about 40 rows.
-static int pick_rows(int n_jobs, int N) {
+// Box height R for n_jobs jobs (one token's) of N rows in items of `boxes` * R: fewest waves of items over the SMs, each wave
+// costing its rows plus a fixed part (pipeline fill and drain) worth about 40 rows.
+static int pick_rows(int n_jobs, int N, int boxes) {
     int best = 128; long best_cost = -1;
     for (int R = 128; R >= 32; R -= 8) {
-        const long tasks = (long)n_jobs * ((N + R - 1) / R), waves = (tasks + sm_count() - 1) / sm_count();
+        const long tasks = (long)n_jobs * ((N + boxes * R - 1) / (boxes * R)), waves = (tasks + sm_count() - 1) / sm_count();
         const long cost = waves * (R + 40);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = R; }
     }
     return best;
-}
-
-__global__ void k_moe_plan(const __grid_constant__ MoePlan q, const int32_t* __restrict__ sel, int M) {
-    const int pair = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pair >= M * q.ns) return;
-    const int m = pair / q.ns, slot = pair - m * q.ns;
-    moe_plan_pair(q, m, slot, slot < q.topk ? sel[(size_t)m * q.topk + slot] : 0);
 }
 
 // y[m, h] = sum over the routed slots in slot order of wts[m, k] * part[row(m, k), h], plus the shared expert's
@@ -93,6 +87,8 @@ k_moe_combine(float* __restrict__ y, const float* __restrict__ part, const float
     __shared__ float w[MC_MAX_SLOTS];
     __shared__ int row[MC_MAX_SLOTS];
     const int m = blockIdx.y, per = H >> 2, i = blockIdx.x * 256 + threadIdx.x;      // float4 index within the token
+    pdl_launch_dependents();
+    pdl_wait();
     if (threadIdx.x < ns) {
         w[threadIdx.x] = threadIdx.x < topk ? wts[(size_t)m * topk + threadIdx.x] : 1.f;
         row[threadIdx.x] = posof ? posof[m * ns + threadIdx.x] : m * ns + threadIdx.x;
@@ -120,7 +116,8 @@ static int combine_launch(float* y, const float* part, const float* wts, const i
     for (int m0 = 0; m0 < M; m0 += 65535) {              // gridDim.y
         const int c = std::min(M - m0, 65535);
         const float* pt = posof ? part : part + (size_t)m0 * ns * H;
-        k_moe_combine<<<dim3(((H >> 2) + 255) / 256, c), 256, 0, s>>>(y + (size_t)m0 * H, pt, wts + (size_t)m0 * topk, posof ? posof + (size_t)m0 * ns : nullptr, c, topk, ns, H);
+        if (launch_pdl(k_moe_combine, dim3(((H >> 2) + 255) / 256, c), 256, 0, s, y + (size_t)m0 * H, pt, wts + (size_t)m0 * topk,
+                       posof ? posof + (size_t)m0 * ns : nullptr, c, topk, ns, H) != cudaSuccess) return launch_failed("k_moe_combine");
         if (int rc = check_launch("k_moe_combine")) return rc;
     }
     return B200_OK;
@@ -134,7 +131,7 @@ static int combine_launch(float* y, const float* part, const float* wts, const i
 constexpr int MG_MAX_GROUPS = 513;                   // n_expert <= 512, plus the shared expert
 
 __global__ void __launch_bounds__(1024)
-k_moe_group(const __grid_constant__ MoePlan q, const int32_t* __restrict__ sel, int* __restrict__ posof,
+k_moe_group(const __grid_constant__ MoePlan q, UmJob* __restrict__ j1, UmJob* __restrict__ j2, const int32_t* __restrict__ sel, int* __restrict__ posof,
             const float* __restrict__ xg, SplitJob* __restrict__ s1, SplitJob* __restrict__ s2,
             unsigned char* __restrict__ img1, unsigned char* __restrict__ img2, float* __restrict__ gam1,
             float* __restrict__ gam2, int M, int max_jobs, unsigned long long* __restrict__ credit_jobs) {
@@ -177,14 +174,14 @@ k_moe_group(const __grid_constant__ MoePlan q, const int32_t* __restrict__ sel, 
             float* ga2 = gam2 + (size_t)idx * 64;
             s1[idx] = SplitJob{xg + pos0 * q.H, nullptr, b1, ga1, rows, 0};
             s2[idx] = SplitJob{g, u, b2, ga2, rows, 0};
-            q.j1[2 * idx] = UmJob{g, nullptr, nullptr, mats[0].gscale, mp, mp + 128, b1, ga1, q.I, rows, 0, 0};
-            q.j1[2 * idx + 1] = UmJob{u, nullptr, nullptr, mats[1].gscale, mp + 256, mp + 384, b1, ga1, q.I, rows, 0, 0};
-            q.j2[idx] = UmJob{q.part + pos0 * q.H, nullptr, nullptr, mats[2].gscale, mp + 512, mp + 640, b2, ga2, q.H, rows, 0, 0};
+            j1[2 * idx] = UmJob{g, nullptr, mats[0].gscale, mp, mp + 128, b1, ga1, q.I, rows, 0, 0};
+            j1[2 * idx + 1] = UmJob{u, nullptr, mats[1].gscale, mp + 256, mp + 384, b1, ga1, q.I, rows, 0, 0};
+            j2[idx] = UmJob{q.part + pos0 * q.H, nullptr, mats[2].gscale, mp + 512, mp + 640, b2, ga2, q.H, rows, 0, 0};
         }
     }
     for (int idx = total_jobs + threadIdx.x; idx < max_jobs; idx += blockDim.x) {
-        const UmJob none{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 0};
-        q.j1[2 * idx] = none; q.j1[2 * idx + 1] = none; q.j2[idx] = none;
+        const UmJob none{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 0};
+        j1[2 * idx] = none; j1[2 * idx + 1] = none; j2[idx] = none;
         s1[idx] = SplitJob{nullptr, nullptr, nullptr, nullptr, 0, 0}; s2[idx] = s1[idx];
     }
 }
@@ -203,15 +200,16 @@ static size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
 static int grouped_max_jobs(const b200_moe_layer* L, int M) { return (M * (L->topk + 1) + 7) / 8 + L->n_expert + 1; }
 
-// Scratch of the tensor-core path behind the logits.  Up to 8 tokens: job tables | gate products |
-// up products | down products, one row per (token, slot) pair.  More: pair positions | job tables |
+// Scratch of the tensor-core path behind the logits.  Up to 8 tokens: job tables and digit weights | SwiGLU rows |
+// their digits | down products, one row per (token, slot) pair; the digits of the token rows lie under the down
+// products, which the gate and up launch has read them before.  More: pair positions | job tables |
 // gathered activations | gate | up | down products, rows grouped by expert.
 static size_t moe_gx_ws_bytes(const b200_moe_layer* L, int M);
 size_t moe_umma_ws_bytes(const b200_moe_layer* L, int M) {
     const size_t ns = (size_t)L->topk + 1, pairs = (size_t)M * ns;
     size_t small = 0;
     if (M <= MU_MAX_TOKENS)
-        small = std::max(moe_gx_ws_bytes(L, M), up256(pairs * 3 * sizeof(UmJob)) + 2 * up256(pairs * L->inter * 4) + up256(pairs * L->hidden * 4));
+        small = std::max(moe_gx_ws_bytes(L, M), up256(pairs * MS_PAIR_BYTES) + 2 * up256(pairs * L->inter * 4) + up256(pairs * L->hidden * 4));
     const size_t mj = (size_t)grouped_max_jobs(L, M);
     return std::max(std::max(small, moe_gx_ws_bytes(L, M)), up256(pairs * 4) + up256(mj * 3 * sizeof(UmJob)) + 2 * up256(mj * sizeof(SplitJob)) + 2 * up256(mj * 64 * 4) +
            up256(mj * (L->hidden >> 8) * 8192) + up256(mj * (L->inter >> 8) * 8192) +
@@ -227,12 +225,13 @@ int moe_umma_plan_args(const float* x, const b200_moe_layer* L, void* scratch, i
     const Prepared* P = &Pc;
     const int ns = L->topk + (L->shared ? 1 : 0), pairs = M * ns, H = L->hidden, I = L->inter;
     char* w = static_cast<char*>(scratch);
-    q->j1 = reinterpret_cast<UmJob*>(w);
-    q->j2 = q->j1 + (size_t)2 * pairs;
-    w += up256((size_t)M * (L->topk + 1) * 3 * sizeof(UmJob));
+    q->j1 = reinterpret_cast<MsJob*>(w);
+    q->j2 = q->j1 + pairs;
+    q->gam1 = reinterpret_cast<float*>(q->j2 + pairs); q->gam2 = q->gam1 + (size_t)M * UM_NB;
+    w += up256((size_t)M * (L->topk + 1) * MS_PAIR_BYTES);
     q->gbuf = reinterpret_cast<float*>(w); w += up256((size_t)M * (L->topk + 1) * I * 4);
-    q->ubuf = reinterpret_cast<float*>(w); w += up256((size_t)M * (L->topk + 1) * I * 4);
-    q->part = reinterpret_cast<float*>(w);
+    q->img2 = reinterpret_cast<unsigned char*>(w); w += up256((size_t)M * (L->topk + 1) * I * 4);
+    q->part = reinterpret_cast<float*>(w); q->img1 = reinterpret_cast<unsigned char*>(w);
     q->experts = L->experts; q->shared = L->shared; q->maps = P->maps; q->x = x;
     q->topk = L->topk; q->ns = ns; q->E = L->n_expert; q->H = H; q->I = I;
     *R_gu = P->R_gu; *R_d = P->R_d;
@@ -252,7 +251,7 @@ static int moe_umma_grouped(const float* x, const b200_moe_layer* L, float* y, c
     char* w = static_cast<char*>(scratch);
     int* posof = reinterpret_cast<int*>(w); w += up256(np * 4);
     MoePlan q{};
-    q.j1 = reinterpret_cast<UmJob*>(w); q.j2 = q.j1 + (size_t)2 * max_jobs; w += up256((size_t)max_jobs * 3 * sizeof(UmJob));
+    UmJob* j1 = reinterpret_cast<UmJob*>(w); UmJob* j2 = j1 + (size_t)2 * max_jobs; w += up256((size_t)max_jobs * 3 * sizeof(UmJob));
     SplitJob* s1 = reinterpret_cast<SplitJob*>(w); w += up256((size_t)max_jobs * sizeof(SplitJob));
     SplitJob* s2 = reinterpret_cast<SplitJob*>(w); w += up256((size_t)max_jobs * sizeof(SplitJob));
     float* gam1 = reinterpret_cast<float*>(w); w += up256((size_t)max_jobs * 64 * 4);
@@ -266,15 +265,15 @@ static int moe_umma_grouped(const float* x, const b200_moe_layer* L, float* y, c
     q.experts = L->experts; q.shared = L->shared; q.maps = P->maps; q.x = x;
     q.topk = L->topk; q.ns = ns; q.E = L->n_expert; q.H = H; q.I = I;
     if (credit_on()) credit_grouped_geometry(H, I);
-    k_moe_group<<<1, 1024, 0, s>>>(q, sel, posof, xg, s1, s2, img1, img2, gam1, gam2, M, max_jobs, credit_on() ? credit_counters() : nullptr);
+    k_moe_group<<<1, 1024, 0, s>>>(q, j1, j2, sel, posof, xg, s1, s2, img1, img2, gam1, gam2, M, max_jobs, credit_on() ? credit_counters() : nullptr);
     if (int rc = check_launch("k_moe_group")) return rc;
     const size_t n4 = (size_t)pairs * (H >> 2);
     k_moe_gather<<<(unsigned)((n4 + 255) / 256), 256, 0, s>>>(xg, x, posof, pairs, ns, H);
     if (int rc = check_launch("k_moe_gather")) return rc;
     if (int rc = umma_split_launch(s1, max_jobs, H, 0.f, s)) return rc;
-    if (int rc = umma_table_launch(q.j1, 2 * max_jobs, I, H, P->R_gu, 0.f, 8, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
+    if (int rc = umma_table_launch(j1, 2 * max_jobs, I, H, P->R_gu, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
     if (int rc = umma_split_launch(s2, max_jobs, I, L->swiglu_limit, s)) return rc;
-    if (int rc = umma_table_launch(q.j2, max_jobs, H, I, P->R_d, L->swiglu_limit, 8, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
+    if (int rc = umma_table_launch(j2, max_jobs, H, I, P->R_d, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
     return combine_launch(y, q.part, wts, posof, M, q.topk, ns, H, s);
 }
 
@@ -392,7 +391,8 @@ static int moe_gx_grouped(const float* x, const b200_moe_layer* L, float* y, con
     q.topk = L->topk; q.ns = ns; q.E = L->n_expert; q.H = H; q.I = I;
     if (credit_on()) credit_grouped_geometry(H, I);
     const int ctas = std::max(1, std::min(16, M / 64)), per = (M + ctas - 1) / ctas;
-    k_moe_group_gx<<<ctas, 1024, 0, s>>>(q, sel, pos, sfrow, sfpos, j1, j2, n_jobs, sf1, sf2, gs1, gs2, M, NT, per, credit_on() ? credit_counters() : nullptr);
+    if (launch_pdl(k_moe_group_gx, ctas, 1024, 0, s, q, sel, pos, sfrow, sfpos, j1, j2, n_jobs, sf1, sf2, gs1, gs2, M, NT, per,
+                   credit_on() ? credit_counters() : nullptr) != cudaSuccess) return launch_failed("k_moe_group_gx");
     if (int rc = check_launch("k_moe_group_gx")) return rc;
     if (int rc = quant_act_launch(1, x, M, H, ActQuant{xq1, sf1, gs1, pos, sfrow, ns, NT, nblk}, s)) return rc;
     if (int rc = gemm_mxf4_table(j1, n_jobs, NT, I, H, true, L->swiglu_limit, xq1, (size_t)pairs, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
@@ -417,12 +417,9 @@ int moe_umma_experts(const float* x, const b200_moe_layer* L, float* y, const in
     const int pairs = M * q.ns;
     credit(B200_CREDIT_MOE_ACT, (double)pairs * 2.0 * q.I * q.H * 0.5625);      // every pair streams its expert (reference kernels/moe.cu:719-722)
     credit(B200_CREDIT_MOE_DOWN, (double)pairs * 1.0 * q.I * q.H * 0.5625);
-    if (!planned) {
-        k_moe_plan<<<(pairs + 127) / 128, 128, 0, s>>>(q, sel, M);
-        if (int rc = check_launch("k_moe_plan")) return rc;
-    }
-    if (int rc = umma_table_launch(q.j1, 2 * pairs, q.I, q.H, R_gu, 0.f, 1, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
-    if (int rc = umma_table_launch(q.j2, pairs, q.H, q.I, R_d, L->swiglu_limit, 1, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
+    if (!planned)
+        if (int rc = moe_stream_plan_launch(q, sel, M, s)) return rc;
+    if (int rc = moe_stream_launch(q, M, R_gu, R_d, L->swiglu_limit, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
     return combine_launch(y, q.part, wts, nullptr, M, q.topk, q.ns, q.H, s);
 }
 
@@ -447,8 +444,8 @@ extern "C" int b200_moe_prepare(const b200_moe_layer* L) {
     Prepared P{};
     P.experts = L->experts; P.shared = L->shared; P.E = E; P.H = L->hidden; P.I = L->inter;
     const int ns = L->topk + (L->shared ? 1 : 0);
-    P.R_gu = pick_rows(2 * ns, L->inter);
-    P.R_d = pick_rows(ns, L->hidden);
+    P.R_gu = pick_rows(ns, L->inter, 1);
+    P.R_d = pick_rows(ns, L->hidden, 2);
     std::vector<unsigned char> host((size_t)nexp * 12 * 128);
     for (int e = 0; e < nexp; ++e) {
         const b200_nvfp4_mat* m = &mats[(size_t)e * 3];

@@ -80,14 +80,6 @@ __global__ void k_finish_gs(float* gs) {
     gs[0] = gs_of_bits(__float_as_uint(gs[0]));
 }
 
-__device__ __forceinline__ void unpack_bf16x16(const uint4& a, const uint4& b, float (&v)[16]) {
-    const uint32_t u[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        v[2 * j] = __uint_as_float(u[j] << 16);
-        v[2 * j + 1] = __uint_as_float(u[j] & 0xffff0000u);
-    }
-}
 __device__ __forceinline__ void store_group(uint8_t* packed, uint8_t* scale, size_t g, uint32_t lo, uint32_t hi, int code, bool vec_out) {
     if (vec_out) {
         reinterpret_cast<uint2*>(packed)[g] = make_uint2(lo, hi);
@@ -122,15 +114,17 @@ k_quantize(const __nv_bfloat16* __restrict__ w, size_t n_groups, const float* __
     }
     for (; g < n_groups; g += stride) {
         const size_t gr = vec_in ? n_groups - 1 - g : g;
-        float v[16];
+        uint32_t u[8];
         if (vec_in) {
-            unpack_bf16x16(reinterpret_cast<const uint4*>(w)[2 * gr], reinterpret_cast<const uint4*>(w)[2 * gr + 1], v);
+            const uint4 a = reinterpret_cast<const uint4*>(w)[2 * gr], b = reinterpret_cast<const uint4*>(w)[2 * gr + 1];
+            u[0] = a.x; u[1] = a.y; u[2] = a.z; u[3] = a.w; u[4] = b.x; u[5] = b.y; u[6] = b.z; u[7] = b.w;
         } else {
+            const unsigned short* h = reinterpret_cast<const unsigned short*>(w) + 16 * gr;
             #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = __bfloat162float(w[16 * gr + j]);
+            for (int j = 0; j < 8; ++j) u[j] = (uint32_t)h[2 * j] | ((uint32_t)h[2 * j + 1] << 16);
         }
         uint32_t lo, hi; int code;
-        quantize_group(v, gs, lo, hi, code);
+        quantize_group_bf16(u, gs, lo, hi, code);
         store_group(packed, scale, gr, lo, hi, code, vec_out);
     }
 }

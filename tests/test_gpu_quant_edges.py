@@ -60,3 +60,41 @@ def test_quantize_with_unaligned_outputs(N, K, off):
     p, s, gs = O.quantize_tensor(O.bf16_bits_to_f32(bits))
     gp, gsc, ggs = W.numpy()
     assert np.array_equal(gp, p) and np.array_equal(gsc, s) and ggs.view(np.uint32)[0] == gs.view(np.uint32)[0]
+
+
+@pytest.mark.parametrize('exp', [0, 20, -20])
+@pytest.mark.parametrize('off', list(range(-12, 13, 2)) + [7, 9])
+def test_bf16_elements_next_to_mid_points(off, exp):
+    """Steps a few ulps off a short mantissa, so that mid-points times the step lie that close to bf16 numbers: where the one
+    conversion per element hands over to the comparisons, and just outside."""
+    P, O = pkg(), oracle()
+    rng, N, K = np.random.default_rng(off + 100), 16, 512
+    gs = np.array([(np.float32(2.0 ** -exp).view(np.int32) + off)], np.int32).view(np.float32)
+    x = (rng.choice(np.concatenate([MID, [0, 0.5, 1, 6]]), (N, K // 16, 16)) * rng.choice([-1, 1], (N, K // 16, 16)) *
+         rng.choice([1, 1.125, 1.5, 2, 3.25, 448], (N, K // 16, 1)) * 2.0 ** exp)
+    x[:, :, 3] = 6 * np.abs(x).max(-1) / 6
+    bits = O.f32_to_bf16_bits(x.astype(np.float32).reshape(N, K))
+    bits = (bits.astype(np.int32) + rng.integers(-1, 2, bits.shape) * (rng.random(bits.shape) < 0.3)).clip(0, 0xffff).astype(bits.dtype)
+    bits[(bits & 0x7f80) == 0x7f80] = 0
+    W = P.quantize(to_dev_bf16(bits), gscale_in=torch.from_numpy(gs).cuda())
+    p, s = O.quantize(O.bf16_bits_to_f32(bits), gs[0])
+    assert np.array_equal(W.packed.cpu().numpy(), p) and np.array_equal(W.scale.cpu().numpy(), s)
+
+
+@pytest.mark.parametrize('off', [0, 1])
+def test_nan_weights_keep_their_zero_code(off):
+    """A NaN exceeds no mid-point: code 0, its neighbours unaffected; aligned and unaligned rows, an odd number of groups."""
+    P, O = pkg(), oracle()
+    N, K = 3, 1040
+    x = np.random.default_rng(8).normal(0, 0.02, (N, K)).astype(np.float32)
+    bits = O.f32_to_bf16_bits(x)
+    where = np.zeros((N, K), bool); where[0, 5] = where[1, 1030] = where[2, K - 1] = where[0, 0] = True
+    clean = bits.copy(); clean[where] = 0
+    bits[where] = 0x7fc0
+    buf = torch.empty(N * K + 8, dtype=torch.bfloat16, device='cuda')
+    w = buf[off:off + N * K].view(N, K)
+    w.copy_(to_dev_bf16(bits))
+    W = P.quantize(w)
+    p, s, gs = O.quantize_tensor(O.bf16_bits_to_f32(clean))
+    gp, gsc, ggs = W.numpy()
+    assert np.array_equal(gp, p) and np.array_equal(gsc, s) and ggs.view(np.uint32)[0] == gs.view(np.uint32)[0]
