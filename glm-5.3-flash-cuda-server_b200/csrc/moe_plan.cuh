@@ -5,10 +5,10 @@
 
 namespace b200 {
 
-// One activation row against one expert matrix, or its gate and its up matrix (moe_stream.cu).  img: the row's digits
-// [K/256][8 digits][128 B], gam: their weights.  mw, mw2: tensor maps of packed weights in GLOBAL memory; sc, sc2: their scales.
+// One activation row against one expert matrix, or its gate and its up matrix (moe_stream.cu).  row: gate and up, the row's
+// digits [K/256][8 digits][128 B], gam their weights; down, the fp32 row itself.  mw, mw2: tensor maps of packed weights in GLOBAL memory; sc, sc2: their scales.
 struct MsJob { float* y; const float* gs; const float* gs2; const void* mw; const void* mw2; const unsigned char* sc;
-               const unsigned char* sc2; const unsigned char* img; const float* gam; };
+               const unsigned char* sc2; const void* row; const float* gam; };
 
 // Where the job tables, the per-expert tensor maps and the intermediate buffers of one call live.
 // maps == nullptr: no plan wanted.
@@ -17,8 +17,7 @@ struct MoePlan {
     const b200_nvfp4_mat* experts; const b200_nvfp4_mat* shared;
     const unsigned char* maps;                     // [(E + 1) experts][gate w,s | up w,s | down w,s] x 128 bytes
     const float* x; float* gbuf; float* ubuf; float* part;
-    unsigned char* img1; unsigned char* img2;      // digits of the token rows and of the SwiGLU rows
-    float* gam1; float* gam2;
+    unsigned char* img1; float* gam1;              // digits of the token rows
     int topk, ns, E, H, I;
 };
 
@@ -33,7 +32,7 @@ __device__ __forceinline__ void moe_plan_pair(const MoePlan& q, int m, int slot,
     q.j1[pair] = MsJob{q.gbuf + (size_t)pair * q.I, g.gscale, u.gscale, mp, mp + 256, g.scale, u.scale,
                        q.img1 + (size_t)m * q.H * 4, q.gam1 + m * UM_NB};
     q.j2[pair] = MsJob{q.part + (size_t)pair * q.H, d.gscale, nullptr, mp + 512, nullptr, d.scale, nullptr,
-                       q.img2 + (size_t)pair * q.I * 4, q.gam2 + pair * UM_NB};
+                       q.gbuf + (size_t)pair * q.I, nullptr};
 }
 
 // Token m's row into digits, by UM_WORKERS threads (t = 0 .. UM_WORKERS - 1).

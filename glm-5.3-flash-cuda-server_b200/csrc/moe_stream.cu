@@ -1,23 +1,26 @@
 // moe_stream.cu -- the experts of up to eight tokens on a prepared layer: one activation row against one expert matrix
 // (or a gate and an up matrix at once) per job, exact as gemv_umma.cu is and bit for bit its results: the row enters as
-// eight FP4 digit columns (digit_split.cuh), split once beforehand, and a weight row's products are summed in four
-// accumulators by 256-k step, in the same order.
+// eight FP4 digit columns (digit_split.cuh), and a weight row's products are summed in four
+// accumulators by 256-k step, in the same order.  Token rows come split; a SwiGLU row is split by every CTA of the down
+// launch that meets it (96 groups of 16 for a row of 1536, during the MMAs of the item before), because a launch of its own
+// for that stood between the two products with the memory idle (hidden 4096, inter 1536, top-8 and shared: 43.5 us a
+// layer at one token and 87.9 at four with that launch, 41.6 and 86.3 without it).
 //
 // What bounds a MoE layer in decode is not the stream but its gaps: one CTA per row tile, as gemv_umma.cu runs, spends
 // 4-6 us from its job record to its first MMA (split, scale slabs, ring fill) with the SM's memory pipe idle, once per tile
 // (four tokens: four times per launch).  Here one CTA per SM walks items (a job's tile of R gate and R up rows, or 2 R rows of
 // one matrix) and its producers run ahead across items, so the ring never drains:
 //   warp 0      TMA: per step two 128B-swizzled boxes of packed weights [128 B x R]
-//   warp 3      the step's 1 KB of the row's digits (one bulk copy)
+//   warp 3      gate and up: the step's 1 KB of the row's digits (one bulk copy)
 //   warps 4-7   weight scales (umma_mxf4.cuh), and once the unit scales of the digits
 //   warp 1      MMA issuer: per step tcgen05.cp of the weight scales, two x four tcgen05.mma (128 x 8, K = 64 each)
 //   warp 2      allocates / frees TMEM
-//   warps 8-15  epilogue: two groups of four take alternate items, each with its own accumulators; sum of the digits, and
-//               for gate and up the clamped SwiGLU, so that the down launch reads one row and no third launch is needed
+//   warps 8-15  down: the digits of the next item's row, together.  Epilogue: two groups of four take alternate items, each
+//               with its own accumulators; sum of the digits, and for gate and up the clamped SwiGLU, so that the down
+//               launch reads one row
 // The job table is written by the routing kernel.  The down launch reads its table and requests its weights before its
-// dependency wait: it can only start once every CTA of the split launch before it has, those once every CTA of the
-// gate and up launch has passed its own wait (they release their dependents after it), and that wait ended when the
-// routing kernel had.
+// dependency wait: it can only start once every CTA of the gate and up launch has passed its own wait (they release their
+// dependents after it), and that wait ended when the routing kernel had.
 // Every wait is bounded (tma_pipe.cuh).  No cluster launch, no multicast.
 #include "b200_internal.h"
 #include "digit_split.cuh"
@@ -38,6 +41,7 @@ struct MsParams {
     const MsJob* table;
     unsigned int* status;
     int n_jobs, tiles, N, K, R, stages, early;         // early: the table may be read and weights requested before the dependency wait
+    int rows_b;                                        // down: digit rows kept at a time (1 or 2)
     uint32_t a_slot, b_off, ts_off;
     float limit;
 };
@@ -46,7 +50,8 @@ template <bool DUAL>
 __global__ void __launch_bounds__(MS_THREADS, 1)
 k_moe_stream(const __grid_constant__ MsParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ uint64_t full_bar[MS_MAX_STAGES], empty_bar[MS_MAX_STAGES], acc_full[2], acc_empty[2];
+    __shared__ uint64_t full_bar[MS_MAX_STAGES], empty_bar[MS_MAX_STAGES], acc_full[2], acc_empty[2], row_full[2];
+    __shared__ float red[UM_MAX_M][8], row_gam[2][UM_NB];
     __shared__ uint32_t tmem_base_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nst = p.K >> 8, R = p.R, S = p.stages;
@@ -57,10 +62,10 @@ k_moe_stream(const __grid_constant__ MsParams p) {
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     } else if (warp == 1) {
         if (lane < S) {
-            mbar_init(smem_u32(&full_bar[lane]), 4);    // the two producer warps, one scale warp per tile
+            mbar_init(smem_u32(&full_bar[lane]), DUAL ? 4 : 3);     // the producer warps, one scale warp per tile
             mbar_init(smem_u32(&empty_bar[lane]), 1);
         }
-        if (lane < 2) { mbar_init(smem_u32(&acc_full[lane]), 1); mbar_init(smem_u32(&acc_empty[lane]), 4); }
+        if (lane < 2) { mbar_init(smem_u32(&acc_full[lane]), 1); mbar_init(smem_u32(&acc_empty[lane]), 4); mbar_init(smem_u32(&row_full[lane]), 8); }
         mbar_fence_init();
     }
     gx_fence_before();
@@ -75,7 +80,7 @@ k_moe_stream(const __grid_constant__ MsParams p) {
     auto job = [&](int i) {
         const unsigned long long* w = reinterpret_cast<const unsigned long long*>(p.table + (first + i * stride) / p.tiles);
         return MsJob{(float*)__ldcg(w), (const float*)__ldcg(w + 1), (const float*)__ldcg(w + 2), (const void*)__ldcg(w + 3), (const void*)__ldcg(w + 4),
-                     (const unsigned char*)__ldcg(w + 5), (const unsigned char*)__ldcg(w + 6), (const unsigned char*)__ldcg(w + 7), (const float*)__ldcg(w + 8)};
+                     (const unsigned char*)__ldcg(w + 5), (const unsigned char*)__ldcg(w + 6), (const void*)__ldcg(w + 7), (const float*)__ldcg(w + 8)};
     };
     auto row0 = [&](int i) { return (first + i * stride) % p.tiles * nrow; };
 
@@ -107,12 +112,11 @@ k_moe_stream(const __grid_constant__ MsParams p) {
             mbar_wait_spin(empty0 + s * 8, ph, p.status, 10);
             if (++s == S) { s = 0; ph ^= 1; }
         }
-    } else if (warp == 3) {
+    } else if (DUAL && warp == 3) {
         // ---- the row's digits ----
-        if (p.early) pdl_wait();
         int s = 0; uint32_t ph = 1;
         for (int i = 0; i < n_items; ++i) {
-            const unsigned char* img = job(i).img;
+            const unsigned char* img = static_cast<const unsigned char*>(job(i).row);
             for (int it = 0; it < nst; ++it, img += 1024) {
                 mbar_wait_spin(empty0 + s * 8, ph, p.status, 7);
                 if (elect_one()) {
@@ -133,6 +137,8 @@ k_moe_stream(const __grid_constant__ MsParams p) {
         for (int i = 0; i < n_items; ++i) {
             const int buf = i & 1, use = i >> 1;
             if (use > 0) mbar_wait_spin(smem_u32(&acc_empty[buf]), (use - 1) & 1, p.status, 14);
+            const int rb = p.rows_b == 2 ? buf : 0;
+            if (!DUAL) mbar_wait_spin(smem_u32(&row_full[rb]), (p.rows_b == 2 ? use : i) & 1, p.status, 7);
             for (int it = 0; it < nst; ++it) {
                 mbar_wait_spin(full0 + s * 8, ph, p.status, 11);
                 gx_fence_after();
@@ -143,7 +149,7 @@ k_moe_stream(const __grid_constant__ MsParams p) {
                         #pragma unroll
                         for (int t = 0; t < 2; ++t)
                             gx_cp_sf(slot + t * 16 + kb * 4, dT0 + (uint64_t)((s * 2 + t) * 128 + kb * 32));
-                    const uint64_t dB = dB0 + (uint64_t)(s * 64);
+                    const uint64_t dB = dB0 + (uint64_t)((DUAL ? s : rb * nst + it) * 64);
                     #pragma unroll
                     for (int t = 0; t < 2; ++t) {
                         const uint64_t dA = dA0 + (uint64_t)(((uint32_t)(s * 2 + t) * p.a_slot) >> 4);
@@ -185,13 +191,26 @@ k_moe_stream(const __grid_constant__ MsParams p) {
         if (p.early) pdl_wait();
         const int grp = (warp - 8) >> 2, q4 = warp & 3, r = q4 * 32 + lane;
         const uint32_t tq = tmem + ((uint32_t)(q4 * 32) << 16);
-        for (int i = grp; i < n_items; i += 2) {
+        // Item i's row into digits.  Its place is free once the MMAs of the last item there are done; both groups wait for
+        // that, and none can fall two phases behind because no later item starts before both have split its row.
+        auto split = [&](int i) {
+            const int rb = p.rows_b == 2 ? i & 1 : 0, last = i - p.rows_b;
+            if (last >= 0) mbar_wait_spin(smem_u32(&acc_full[last & 1]), (last >> 1) & 1, p.status, 8);
+            split_rows<true>(static_cast<const float*>(job(i).row), nullptr, 0.f, 1, p.K, 1, ring + p.b_off + (size_t)rb * nst * 1024, row_gam[rb], red, tid - 256);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // generic-proxy stores -> the MMA's async-proxy reads
+            named_sync(1, UM_WORKERS);
+            if (lane == 0) mbar_arrive(smem_u32(&row_full[rb]));
+        };
+        if (!DUAL && n_items) split(0);
+        for (int i = 0; i < n_items; ++i) {
+            if (!DUAL && p.rows_b == 2 && i + 1 < n_items) split(i + 1);
+            if ((i & 1) != grp) continue;
             const MsJob J = job(i);
             const int use = i >> 1, row = row0(i) + r;
             const float gs0 = J.gs[0], gs1 = DUAL ? J.gs2[0] : gs0;
             float gam[UM_NB];
             #pragma unroll
-            for (int d = 0; d < UM_NB; ++d) gam[d] = __ldcg(J.gam + d);
+            for (int d = 0; d < UM_NB; ++d) gam[d] = DUAL ? __ldcg(J.gam + d) : row_gam[p.rows_b == 2 ? grp : 0][d];
             float* y = J.y;
             mbar_wait_spin(smem_u32(&acc_full[grp]), use & 1, p.status, 14);
             gx_fence_after();
@@ -234,16 +253,6 @@ k_moe_stream(const __grid_constant__ MsParams p) {
     if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(MS_TMEM_COLS));
 }
 
-// One CTA per pair: its SwiGLU row into the digits the down launch reads.
-__global__ void __launch_bounds__(UM_WORKERS)
-k_split_act(const __grid_constant__ MoePlan q) {
-    __shared__ float red[UM_MAX_M][8];
-    pdl_launch_dependents();
-    pdl_wait();
-    const size_t pair = blockIdx.x;
-    split_rows<true>(q.gbuf + pair * q.I, nullptr, 0.f, 1, q.I, 1, q.img2 + pair * q.I * 4, q.gam2 + pair * UM_NB, red, (int)threadIdx.x);
-}
-
 // The job records and the digits of the token rows from selections that are there already.
 __global__ void __launch_bounds__(UM_WORKERS + 32)
 k_moe_plan(const __grid_constant__ MoePlan q, const int32_t* __restrict__ sel) {
@@ -271,12 +280,15 @@ static int stream_launch(const MsJob* table, int n_jobs, int N, int K, int R, fl
     p.tiles = (N + (DUAL ? R : 2 * R) - 1) / (DUAL ? R : 2 * R);
     p.a_slot = ((uint32_t)R * 128u + 1023u) & ~1023u;
     const int items = n_jobs * p.tiles, grid = std::min(items, sm_count()), nst = K / 256;
-    const size_t stage = 2 * (size_t)p.a_slot + 1024 + 2 * 2048;
-    p.stages = (int)std::min<size_t>(std::min<long>((long)((items + grid - 1) / grid) * nst, MS_MAX_STAGES), (ROOM - 1024) / stage);
+    const int per_cta = (items + grid - 1) / grid;
+    // down: whole digit rows, a second one where there is an item to split ahead for; a single item keeps one more stage
+    p.rows_b = per_cta > 1 ? 2 : 1;
+    const size_t stage = 2 * (size_t)p.a_slot + (DUAL ? 1024 : 0) + 2 * 2048, rows = DUAL ? 0 : (size_t)p.rows_b * nst * 1024;
+    p.stages = (int)std::min<size_t>(std::min<long>((long)per_cta * nst, MS_MAX_STAGES), (ROOM - 1024 - rows) / stage);
     // the MMA reads 16 KB from the start of a weight slot whatever R; what lies behind the last one covers that (R >= 32)
     p.b_off = (uint32_t)p.stages * 2 * p.a_slot;
-    p.ts_off = p.b_off + (uint32_t)p.stages * 1024u;
-    const size_t smem = std::max((size_t)p.stages * stage, (size_t)(2 * p.stages - 1) * p.a_slot + 16384) + 1024;
+    p.ts_off = p.b_off + (DUAL ? (uint32_t)p.stages * 1024u : (uint32_t)rows);
+    const size_t smem = std::max((size_t)p.stages * stage + rows, (size_t)(2 * p.stages - 1) * p.a_slot + 16384) + 1024;
     if (p.stages < 1 || smem > ROOM) return B200_ENOTIMPL;
     static bool ready[64] = {};
     int dev = 0;
@@ -300,8 +312,6 @@ int moe_stream_plan_launch(const MoePlan& q, const int32_t* sel, int M, cudaStre
 int moe_stream_launch(const MoePlan& q, int M, int R_gu, int R_d, float limit, cudaStream_t s) {
     const int pairs = M * q.ns;
     if (int rc = stream_launch<true>(q.j1, pairs, q.I, q.H, R_gu, limit, false, s)) return rc;
-    if (launch_pdl(k_split_act, pairs, UM_WORKERS, 0, s, q) != cudaSuccess) return launch_failed("k_split_act");
-    if (int rc = check_launch("k_split_act")) return rc;
     return stream_launch<false>(q.j2, pairs, q.H, q.I, R_d, 0.f, true, s);
 }
 

@@ -28,7 +28,7 @@
 namespace b200 {
 
 constexpr int MU_MAX_TOKENS = 8;
-constexpr size_t MS_PAIR_BYTES = 2 * sizeof(MsJob) + 2 * UM_NB * sizeof(float);     // two job records, two rows of digit weights
+constexpr size_t MS_PAIR_BYTES = 2 * sizeof(MsJob) + UM_NB * sizeof(float);     // two job records, a row of digit weights
 // Fewest tokens for which the (token, slot) pairs are sorted by expert, so that every distinct expert
 // (and the shared expert) is streamed once for up to 8 rows instead of once per pair (the reference's
 // gathered kernels, kernels/moe.cu:353-581).  Below it every pair is its own job.  B200_MOE_GROUP_MIN
@@ -201,7 +201,7 @@ static size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 static int grouped_max_jobs(const b200_moe_layer* L, int M) { return (M * (L->topk + 1) + 7) / 8 + L->n_expert + 1; }
 
 // Scratch of the tensor-core path behind the logits.  Up to 8 tokens: job tables and digit weights | SwiGLU rows |
-// their digits | down products, one row per (token, slot) pair; the digits of the token rows lie under the down
+// down products, one row per (token, slot) pair; the digits of the token rows lie under the down
 // products, which the gate and up launch has read them before.  More: pair positions | job tables |
 // gathered activations | gate | up | down products, rows grouped by expert.
 static size_t moe_gx_ws_bytes(const b200_moe_layer* L, int M);
@@ -209,7 +209,7 @@ size_t moe_umma_ws_bytes(const b200_moe_layer* L, int M) {
     const size_t ns = (size_t)L->topk + 1, pairs = (size_t)M * ns;
     size_t small = 0;
     if (M <= MU_MAX_TOKENS)
-        small = std::max(moe_gx_ws_bytes(L, M), up256(pairs * MS_PAIR_BYTES) + 2 * up256(pairs * L->inter * 4) + up256(pairs * L->hidden * 4));
+        small = std::max(moe_gx_ws_bytes(L, M), up256(pairs * MS_PAIR_BYTES) + up256(pairs * L->inter * 4) + up256(pairs * L->hidden * 4));
     const size_t mj = (size_t)grouped_max_jobs(L, M);
     return std::max(std::max(small, moe_gx_ws_bytes(L, M)), up256(pairs * 4) + up256(mj * 3 * sizeof(UmJob)) + 2 * up256(mj * sizeof(SplitJob)) + 2 * up256(mj * 64 * 4) +
            up256(mj * (L->hidden >> 8) * 8192) + up256(mj * (L->inter >> 8) * 8192) +
@@ -227,10 +227,9 @@ int moe_umma_plan_args(const float* x, const b200_moe_layer* L, void* scratch, i
     char* w = static_cast<char*>(scratch);
     q->j1 = reinterpret_cast<MsJob*>(w);
     q->j2 = q->j1 + pairs;
-    q->gam1 = reinterpret_cast<float*>(q->j2 + pairs); q->gam2 = q->gam1 + (size_t)M * UM_NB;
+    q->gam1 = reinterpret_cast<float*>(q->j2 + pairs);
     w += up256((size_t)M * (L->topk + 1) * MS_PAIR_BYTES);
     q->gbuf = reinterpret_cast<float*>(w); w += up256((size_t)M * (L->topk + 1) * I * 4);
-    q->img2 = reinterpret_cast<unsigned char*>(w); w += up256((size_t)M * (L->topk + 1) * I * 4);
     q->part = reinterpret_cast<float*>(w); q->img1 = reinterpret_cast<unsigned char*>(w);
     q->experts = L->experts; q->shared = L->shared; q->maps = P->maps; q->x = x;
     q->topk = L->topk; q->ns = ns; q->E = L->n_expert; q->H = H; q->I = I;

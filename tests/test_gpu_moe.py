@@ -241,6 +241,26 @@ def test_moe_grouped_wide_gemm_job_shapes(H, I, E, M, topk, shared):
     test_moe_prefill_widths_run_the_grouped_wide_gemm(H, I, E, M, topk, shared, True)
 
 
+@pytest.mark.parametrize('H,I,topk,M', [(512, 256, 3, 1), (512, 256, 3, 8), (4096, 768, 8, 3), (2048, 8192, 2, 8), (4096, 12288, 1, 8), (256, 16384, 1, 2)])
+def test_moe_decode_down_launch_splits_its_rows(H, I, topk, M):
+    """The down launch splits the SwiGLU row of each item itself: rows of one k-step and of 64 (two stages of
+    ring left), one item per CTA and several, an odd and an even number of them; against the oracle, and every
+    token equal to that token alone, where a CTA has other items, bit for bit."""
+    P = pkg()
+    layer, d = build_layer(H, I, 9, topk, seed=I + M, on_gpu=True)
+    x = np.random.default_rng(M + I).normal(0, 1, (M, H)).astype(np.float32)
+    xd = torch.from_numpy(x).cuda()
+    assert P.moe_prepare(layer)
+    try:
+        y, sel, wts = check_layer(layer, d, x)
+        for m in range(M):
+            assert torch.equal(P.moe_forward(layer, xd[m:m + 1].contiguous())[0][0], y[m]), m
+        for _ in range(20): assert torch.equal(P.moe_forward(layer, xd)[0], y)
+        assert P.device_status() == 0
+    finally:
+        P.moe_release(layer)
+
+
 def test_moe_prepared_layer_under_graph_capture():
     """The prepared path only launches kernels (descriptor look-up is host-side), so a layer forward
     can be captured and replayed; small-batch and grouped paths."""
