@@ -16,12 +16,14 @@
 //   warp 0      TMA: per super-step the packed weights [128 B x 128 rows] (128B-swizzled) and their scale bytes
 //               [16 B x 128 rows] into one slot of a ring
 //   warp 3      TMA: per half-step two boxes [128 B x NT rows] of the fp16 activations (64 k each)
-//   warps 4-11  converters: per half-step 128 rows x 128 k: cvt.rn.f16x2.e2m1x2, times the group's scale
-//               (e4m3 -> f16, exact), stored as the K-major 128B-swizzled fp16 tile the MMA reads; several
-//               operand buffers, so that the conversion runs ahead of the MMAs
+//   warps 4-15  converters, three groups of four taking every third half-step (128 rows x 128 k, a thread a row):
+//               cvt.rn.f16x2.e2m1x2, times the group's scale (e4m3 -> f16, exact), kept in registers until an operand
+//               buffer is free, then stored as the K-major 128B-swizzled fp16 tile the MMA reads
 //   warp 1      MMA issuer: 8 tcgen05.mma.kind::f16 (K = 16 each) per half-step, tcgen05.commit frees
 //               the operand buffer, the activation slot and (every second half-step) the packed slot
-//   warp 2      TMEM allocation;  warps 12-15  epilogue: D[128 rows, NT tokens] * 2^e[token] / gs_w -> y
+//   warp 2      TMEM allocation;  warps 12-15  at the end the epilogue: D[128 rows, NT tokens] * 2^e[token] / gs_w -> y
+// [4096 x 4096]: 16 rows 25.4 us with one group of eight converter warps, 22.5 so; 300 rows 31.5 and 28.4; [12288 x 4096] x 1024
+// rows 175 and 166 (of each about 2 us are k_act_f16, eight elements a load instead of one).
 // Barriers are per step and used once (K <= 16384: 64 super-steps, 128 half-steps); every wait is bounded.
 // No cluster launch, no multicast.
 #include "b200_internal.h"
@@ -34,7 +36,7 @@
 namespace b200 {
 
 constexpr int GF_THREADS = 512;
-constexpr int GF_CONV = 256;
+constexpr int GF_GROUPS = 3, GF_GROUP_WARPS = 4;              // converters; warps 4 .. 15
 constexpr int GF_MAX_SUPER = 64, GF_MAX_HALF = 128;          // K <= 16384
 constexpr uint32_t GF_P_BYTES = 16384 + 2048;                // a super-step: packed weights 128 rows x 128 B, then their scales 128 rows x 16 B
 constexpr uint32_t GF_A16_BYTES = 32768;                     // fp16 operand of a half-step: 2 k-blocks x [128 rows x 128 B]
@@ -75,7 +77,7 @@ k_gemm_f16w(const __grid_constant__ GfParams p, const __grid_constant__ CUtensor
     for (int i = tid; i < nsup; i += GF_THREADS) mbar_init(smem_u32(&fullP[i]), 1);
     for (int i = tid; i < nhalf; i += GF_THREADS) {
         mbar_init(smem_u32(&fullB[i]), 1);
-        mbar_init(smem_u32(&a16_full[i]), GF_CONV / 32);
+        mbar_init(smem_u32(&a16_full[i]), GF_GROUP_WARPS);
         mbar_init(smem_u32(&done16[i]), 1);
     }
     if (tid == 0) mbar_init(smem_u32(&done_bar), 1);
@@ -97,9 +99,12 @@ k_gemm_f16w(const __grid_constant__ GfParams p, const __grid_constant__ CUtensor
         }
         if (!p.prefetch_before_wait) pdl_wait();
         for (int g = 0, sl = 0; g < nsup; ++g) {
-            // the slot is free once the operand of the second half-step of the super-step that held it has been
-            // converted (a16_full), not only multiplied: the MMAs never read the packed bytes
-            if (g >= p.sp) mbar_wait_spin(smem_u32(&a16_full[2 * (g - p.sp) + 1]), 0, p.status, 21);
+            // the slot is free once both half-steps of the super-step that held it have been converted (a16_full; by two
+            // groups, in either order), not only multiplied: the MMAs never read the packed bytes
+            if (g >= p.sp) {
+                mbar_wait_spin(smem_u32(&a16_full[2 * (g - p.sp)]), 0, p.status, 21);
+                mbar_wait_spin(smem_u32(&a16_full[2 * (g - p.sp) + 1]), 0, p.status, 21);
+            }
             if (elect_one()) {
                 const uint32_t bar = smem_u32(&fullP[g]), dst = smem_u32(ringP) + (uint32_t)sl * GF_P_BYTES;
                 mbar_expect_tx(bar, GF_P_BYTES);
@@ -156,57 +161,62 @@ k_gemm_f16w(const __grid_constant__ GfParams p, const __grid_constant__ CUtensor
         }
         if (elect_one()) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(&done_bar)) : "memory");
         __syncwarp();
-    } else if (warp >= 4 && warp < 12) {
-        // ---- converters: thread -> (weight row r, k-block kb of the half-step) ----
-        const int t = tid - 128, r = t & 127, kb = t >> 7;      // a quarter-warp = 8 consecutive rows: conflict-free swizzled accesses
-        for (int h = 0; h < nhalf; ++h) {
+    } else if (warp >= 4) {
+        // ---- converters: thread -> weight row r of its group's half-steps ----
+        const int r = (tid & 127), grp = (warp - 4) / GF_GROUP_WARPS;      // a quarter-warp = 8 consecutive rows: conflict-free swizzled accesses
+        for (int h = grp; h < nhalf; h += GF_GROUPS) {
             const int g = h >> 1, half = h & 1;
             mbar_wait_spin(smem_u32(&fullP[g]), 0, p.status, 27);
-            if (h >= p.na) mbar_wait_spin(smem_u32(&done16[h - p.na]), 0, p.status, 28);      // the operand buffer is free again
-            const unsigned char* pk = ringP + (size_t)(g % p.sp) * GF_P_BYTES + (size_t)r * 128;
-            const int j0 = half * 4 + kb * 2;
-            const uint4 w0 = *reinterpret_cast<const uint4*>(pk + (((j0) ^ (r & 7)) << 4));
-            const uint4 w1 = *reinterpret_cast<const uint4*>(pk + (((j0 + 1) ^ (r & 7)) << 4));
-            const uint32_t sc4 = *reinterpret_cast<const uint32_t*>(ringP + (size_t)(g % p.sp) * GF_P_BYTES + 16384 + r * 16 + half * 8 + kb * 4);      // four group scales
-            const uint32_t s01 = e4m3x2_to_h2((uint16_t)(sc4 & 0xffffu)), s23 = e4m3x2_to_h2((uint16_t)(sc4 >> 16));
-            const uint32_t sc[4] = {__byte_perm(s01, s01, 0x1010), __byte_perm(s01, s01, 0x3232), __byte_perm(s23, s23, 0x1010), __byte_perm(s23, s23, 0x3232)};
-            const uint32_t w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-            unsigned char* dst = a16 + (size_t)(h % p.na) * GF_A16_BYTES + (size_t)kb * 16384 + (size_t)r * 128;
+            const unsigned char* slot = ringP + (size_t)(g % p.sp) * GF_P_BYTES;
+            const unsigned char* pk = slot + (size_t)r * 128;
+            const uint2 sc8 = *reinterpret_cast<const uint2*>(slot + 16384 + r * 16 + half * 8);      // eight group scales
+            uint4 o[16];                             // the row's 128 k
             #pragma unroll
-            for (int q = 0; q < 8; ++q) {            // word q: weights 8q .. 8q+7 of the k-block, group q / 2
-                uint32_t hh[4];
-                e2m1x8_to_h2(w[q], hh);
-                const uint32_t s2 = sc[q >> 1];
-                const uint4 o = make_uint4(hmul2_u(hh[0], s2), hmul2_u(hh[1], s2), hmul2_u(hh[2], s2), hmul2_u(hh[3], s2));
-                *reinterpret_cast<uint4*>(dst + ((q ^ (r & 7)) << 4)) = o;
+            for (int c = 0; c < 4; ++c) {            // 32 weights, two groups
+                const uint4 wv = *reinterpret_cast<const uint4*>(pk + (((half * 4 + c) ^ (r & 7)) << 4));
+                const uint32_t w[4] = {wv.x, wv.y, wv.z, wv.w};
+                const uint32_t s2 = e4m3x2_to_h2((uint16_t)(((c & 2) ? sc8.y : sc8.x) >> ((c & 1) * 16)));
+                #pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    uint32_t hh[4];
+                    e2m1x8_to_h2(w[q], hh);
+                    const uint32_t sd = __byte_perm(s2, s2, q < 2 ? 0x1010 : 0x3232);
+                    o[c * 4 + q] = make_uint4(hmul2_u(hh[0], sd), hmul2_u(hh[1], sd), hmul2_u(hh[2], sd), hmul2_u(hh[3], sd));
+                }
             }
+            if (h >= p.na) mbar_wait_spin(smem_u32(&done16[h - p.na]), 0, p.status, 28);      // the operand buffer is free again
+            unsigned char* dst = a16 + (size_t)(h % p.na) * GF_A16_BYTES + (size_t)r * 128;
+            #pragma unroll
+            for (int q = 0; q < 16; ++q)             // k-block q / 8, eight k each
+                *reinterpret_cast<uint4*>(dst + (q >> 3) * 16384 + (((q & 7) ^ (r & 7)) << 4)) = o[q];
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // generic-proxy stores -> the MMA's async-proxy reads
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&a16_full[h]));
         }
-    } else if (warp >= 12) {
-        // ---- epilogue ----
-        const int te = tid - 384, q4 = warp & 3;
-        pdl_wait();
-        if (te < NT) sx[te] = te < rows ? p.rowscale[m0 + te] / p.gs_w[0] : 0.f;
-        named_sync(1, 128);
-        mbar_wait_spin(smem_u32(&done_bar), 0, p.status, 29);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t tq = tmem + ((uint32_t)(q4 * 32) << 16);
-        const int row = rown0 + q4 * 32 + lane;
-        #pragma unroll 1
-        for (int c0 = 0; c0 < NT; c0 += 16) {
-            if (c0 >= rows) break;
-            uint32_t d[16];
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]),
-                           "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
-                         : "r"(tq + (uint32_t)c0));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (row < p.N) {
-                #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    if (c0 + j < rows) p.y[(size_t)(m0 + c0 + j) * p.N + row] = __uint_as_float(d[j]) * sx[c0 + j];
+        if (warp >= 12) {
+            // ---- epilogue ----
+            const int te = tid - 384, q4 = warp & 3;
+            pdl_wait();
+            if (te < NT) sx[te] = te < rows ? p.rowscale[m0 + te] / p.gs_w[0] : 0.f;
+            named_sync(1, 128);
+            mbar_wait_spin(smem_u32(&done_bar), 0, p.status, 29);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t tq = tmem + ((uint32_t)(q4 * 32) << 16);
+            const int row = rown0 + q4 * 32 + lane;
+            #pragma unroll 1
+            for (int c0 = 0; c0 < NT; c0 += 16) {
+                if (c0 >= rows) break;
+                uint32_t d[16];
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                             : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]),
+                               "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
+                             : "r"(tq + (uint32_t)c0));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (row < p.N) {
+                    #pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (c0 + j < rows) p.y[(size_t)(m0 + c0 + j) * p.N + row] = __uint_as_float(d[j]) * sx[c0 + j];
+                }
             }
         }
     }
@@ -225,11 +235,31 @@ k_act_f16(const void* __restrict__ xin, int K, __half* __restrict__ xh, float* _
     const int row = blockIdx.x, tid = threadIdx.x;
     pdl_launch_dependents();
     pdl_wait();
-    auto ld = [&](int i) -> float {
-        return F32 ? static_cast<const float*>(xin)[(size_t)row * K + i] : __bfloat162float(static_cast<const __nv_bfloat16*>(xin)[(size_t)row * K + i]);
+    // eight elements at a time (K % 256 == 0, rows 16-byte aligned); the first two of a thread stay in registers
+    auto ld = [&](int c, float (&v)[8]) {
+        if (F32) {
+            const float4* q = reinterpret_cast<const float4*>(static_cast<const float*>(xin) + (size_t)row * K) + 2 * c;
+            const float4 a = q[0], b = q[1];
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        } else {
+            const uint4 a = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(xin) + (size_t)row * K)[c];
+            const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+            #pragma unroll
+            for (int j = 0; j < 4; ++j) { v[2 * j] = __uint_as_float(w[j] << 16); v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u); }
+        }
     };
+    const int nc = K >> 3;
+    float keep[2][8];
     uint32_t ai = 0u;
-    for (int i = tid; i < K; i += 256) ai = max(ai, __float_as_uint(ld(i)) & 0x7fffffffu);
+    auto most = [&](const float (&v)[8]) {
+        #pragma unroll
+        for (int j = 0; j < 8; ++j) ai = max(ai, __float_as_uint(v[j]) & 0x7fffffffu);
+    };
+    #pragma unroll
+    for (int q = 0; q < 2; ++q) if (tid + q * 256 < nc) ld(tid + q * 256, keep[q]);
+    #pragma unroll
+    for (int q = 0; q < 2; ++q) if (tid + q * 256 < nc) most(keep[q]);
+    for (int c = tid + 512; c < nc; c += 256) { float v[8]; ld(c, v); most(v); }
     #pragma unroll
     for (int o = 16; o; o >>= 1) ai = max(ai, __shfl_xor_sync(0xffffffffu, ai, o));
     if ((tid & 31) == 0) red[tid >> 5] = ai;
@@ -243,7 +273,15 @@ k_act_f16(const void* __restrict__ xin, int K, __half* __restrict__ xh, float* _
     const float down = __uint_as_float((uint32_t)min(127 + 13 - e, 254) << 23);           // 2^(13 - e)
     const float sc = (ai == 0u || bad) ? 1.f : down;
     if (tid == 0) rowscale[row] = bad ? __uint_as_float(0x7fc00000u) : 1.f / sc;
-    for (int i = tid; i < K; i += 256) xh[(size_t)row * K + i] = __float2half_rn(ld(i) * sc);
+    auto put = [&](int c, const float (&v)[8]) {
+        __half2 h[4];
+        #pragma unroll
+        for (int j = 0; j < 4; ++j) h[j] = __halves2half2(__float2half_rn(v[2 * j] * sc), __float2half_rn(v[2 * j + 1] * sc));
+        *reinterpret_cast<uint4*>(xh + (size_t)row * K + (size_t)c * 8) = *reinterpret_cast<const uint4*>(h);
+    };
+    #pragma unroll
+    for (int q = 0; q < 2; ++q) if (tid + q * 256 < nc) put(tid + q * 256, keep[q]);
+    for (int c = tid + 512; c < nc; c += 256) { float v[8]; ld(c, v); put(c, v); }
 }
 
 static size_t up256(size_t v) { return (v + 255) / 256 * 256; }

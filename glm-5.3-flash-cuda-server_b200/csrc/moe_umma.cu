@@ -1,4 +1,4 @@
-// moe_umma.cu -- the MoE experts on the tensor-core gemv kernel (gemv_umma.cu), once
+// moe_umma.cu -- the MoE experts on the tensor-core kernels (moe_stream.cu, gemv_umma.cu, gemm_mxf4.cu), once
 // b200_moe_prepare() has been called for the layer.
 //
 // The expert tables of a layer live in device memory and the router picks experts on the device,
@@ -7,9 +7,8 @@
 // scales) and keeps them in device memory; at run time a small kernel turns (token, slot) pairs
 // into job records that point at the maps of the selected experts.
 //
-// Launches per layer: router logits, k_route, k_moe_plan, gate+up products of all pairs (one
-// tensor-core launch), down products (one tensor-core launch; it reads the two products and
-// applies the clamped SwiGLU while it splits its activation vector), k_moe_combine.
+// Launches per layer up to 8 tokens: router logits, k_route (with the job records and the token rows' digits), gate and up
+// with the SwiGLU, down, k_moe_combine (moe_stream.cu).
 // Up to 8 tokens every (token, slot) pair is its own single-row job, the shared expert included
 // (its weights are read once from HBM and then from L2).  Beyond 8 tokens the pairs are sorted by
 // expert on the device and an expert's rows run in chunks of up to 8, each chunk split into its

@@ -225,6 +225,13 @@ def test_gemm_bf16_exact_vs_oracle(M, N, K):
     assert P.device_status() == 0
 
 
+@pytest.mark.parametrize('M,N,K', [(17, 130, 768), (70, 129, 1280), (129, 70, 16384)])
+def test_gemm_bf16_exact_steps_over_converter_groups(M, N, K):
+    """Half-steps that do not divide evenly among the three converter groups, and the longest K (activation rows that
+    a thread does not keep in registers whole)."""
+    test_gemm_bf16_exact_vs_oracle(M, N, K)
+
+
 def test_gemm_bf16_exact_rows_independent_and_repeatable():
     P = pkg()
     W = P.Nvfp4Weight(*host_triple((500, 1024), 77))
