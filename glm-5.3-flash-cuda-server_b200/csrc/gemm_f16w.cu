@@ -12,18 +12,20 @@
 // decode cost is paid once per weight and CTA, not once per weight and row.
 //
 // One CTA of 16 warps per (128 weight rows, job of up to NT activation rows); K in super-steps of 256 (one TMA
-// box of packed weights) = two half-steps of 128 (what the fp16 operand buffers hold).
+// box of packed weights) = two half-steps of 128 (what an fp16 operand buffer, 64 columns of TMEM, holds).
 //   warp 0      TMA: per super-step the packed weights [128 B x 128 rows] (128B-swizzled) and their scale bytes
 //               [16 B x 128 rows] into one slot of a ring
 //   warp 3      TMA: per half-step two boxes [128 B x NT rows] of the fp16 activations (64 k each)
 //   warps 4-15  converters, three groups of four taking every third half-step (128 rows x 128 k, a thread a row):
 //               cvt.rn.f16x2.e2m1x2, times the group's scale (e4m3 -> f16, exact), kept in registers until an operand
-//               buffer is free, then stored as the K-major 128B-swizzled fp16 tile the MMA reads
+//               buffer is free, then stored to tensor memory, from where the MMA takes A: through shared memory the
+//               tile cost 64 KB of its bandwidth per half-step, as much as the activations, and that bounded the kernel
 //   warp 1      MMA issuer: 8 tcgen05.mma.kind::f16 (K = 16 each) per half-step, tcgen05.commit frees
 //               the operand buffer, the activation slot and (every second half-step) the packed slot
 //   warp 2      TMEM allocation;  warps 12-15  at the end the epilogue: D[128 rows, NT tokens] * 2^e[token] / gs_w -> y
-// [4096 x 4096]: 16 rows 25.4 us with one group of eight converter warps, 22.5 so; 300 rows 31.5 and 28.4; [12288 x 4096] x 1024
-// rows 175 and 166 (of each about 2 us are k_act_f16, eight elements a load instead of one).
+// [4096 x 4096], 16 and 300 rows: 25.4 and 31.5 us with one group of eight converter warps, 22.5 and 28.4 with three groups
+// (about 2 us of it k_act_f16, eight elements a load instead of one), 19.5 and 25.7 with A in tensor memory; [12288 x 4096]
+// x 1024 rows 175, 166 and 150.
 // Barriers are per step and used once (K <= 16384: 64 super-steps, 128 half-steps); every wait is bounded.
 // No cluster launch, no multicast.
 #include "b200_internal.h"
@@ -39,7 +41,9 @@ constexpr int GF_THREADS = 512;
 constexpr int GF_GROUPS = 3, GF_GROUP_WARPS = 4;              // converters; warps 4 .. 15
 constexpr int GF_MAX_SUPER = 64, GF_MAX_HALF = 128;          // K <= 16384
 constexpr uint32_t GF_P_BYTES = 16384 + 2048;                // a super-step: packed weights 128 rows x 128 B, then their scales 128 rows x 16 B
-constexpr uint32_t GF_A16_BYTES = 32768;                     // fp16 operand of a half-step: 2 k-blocks x [128 rows x 128 B]
+static_assert(GF_P_BYTES % 1024 == 0, "the activation ring behind the packed slots is a swizzled operand");
+constexpr uint32_t GF_A_COLS = 64;                           // fp16 operand of a half-step in TMEM: a row per lane, two k per column
+constexpr int GF_A_BUFS = 4;
 
 struct GfParams {
     float* y; const float* gs_w; const float* rowscale;      // rowscale[m] = 2^e of token m (NaN for a non-finite token)
@@ -59,6 +63,8 @@ template <int NT>
 __global__ void __launch_bounds__(GF_THREADS, 1)
 k_gemm_f16w(const __grid_constant__ GfParams p, const __grid_constant__ CUtensorMap map_x,
             const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s) {
+    constexpr uint32_t TMEM_COLS = 512;                      // accumulator [0, NT) | operand buffers
+    static_assert(NT + GF_A_BUFS * GF_A_COLS <= TMEM_COLS, "operand buffers");
     constexpr uint32_t B_BYTES = 2u * NT * 128u;             // activations of a half-step: 2 k-blocks x [NT rows x 128 B]
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint64_t fullP[GF_MAX_SUPER], fullB[GF_MAX_HALF], a16_full[GF_MAX_HALF], done16[GF_MAX_HALF], done_bar;
@@ -70,8 +76,7 @@ k_gemm_f16w(const __grid_constant__ GfParams p, const __grid_constant__ CUtensor
     const int rown0 = tile_n * 128, m0 = ji * NT, rows = min(NT, p.M - m0);
 
     unsigned char* ringP = smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);
-    unsigned char* a16 = ringP + (size_t)p.sp * GF_P_BYTES;          // na operand buffers
-    unsigned char* ringB = a16 + (size_t)p.na * GF_A16_BYTES;
+    unsigned char* ringB = ringP + (size_t)p.sp * GF_P_BYTES;
 
     pdl_launch_dependents();
     for (int i = tid; i < nsup; i += GF_THREADS) mbar_init(smem_u32(&fullP[i]), 1);
@@ -83,7 +88,7 @@ k_gemm_f16w(const __grid_constant__ GfParams p, const __grid_constant__ CUtensor
     if (tid == 0) mbar_init(smem_u32(&done_bar), 1);
     mbar_fence_init();
     if (warp == 2) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&tmem_base_s)), "r"(NT < 32 ? 32 : NT));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&tmem_base_s)), "r"(TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -137,22 +142,23 @@ k_gemm_f16w(const __grid_constant__ GfParams p, const __grid_constant__ CUtensor
     } else if (warp == 1) {
         // ---- MMA issuer ----
         const uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((128u >> 4) << 24);     // D f32, A and B f16, K-major
-        const uint64_t dA0 = gf_desc(smem_u32(a16)), dB0 = gf_desc(smem_u32(ringB));
+        const uint64_t dB0 = gf_desc(smem_u32(ringB));
         for (int h = 0; h < nhalf; ++h) {
             mbar_wait_spin(smem_u32(&a16_full[h]), 0, p.status, 24);
             mbar_wait_spin(smem_u32(&fullB[h]), 0, p.status, 25);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (elect_one()) {
-                const uint64_t oA = (uint64_t)(((uint32_t)(h % p.na) * GF_A16_BYTES) >> 4), oB = (uint64_t)(((uint32_t)(h % p.sb) * B_BYTES) >> 4);
+                const uint32_t tA = tmem + NT + (uint32_t)(h % p.na) * GF_A_COLS;
+                const uint64_t oB = (uint64_t)(((uint32_t)(h % p.sb) * B_BYTES) >> 4);
                 #pragma unroll
                 for (int kb = 0; kb < 2; ++kb) {
                     #pragma unroll
                     for (int k16 = 0; k16 < 4; ++k16) {
-                        const uint64_t da = dA0 + oA + (uint64_t)(kb * (16384 >> 4)) + k16 * 2;
+                        const uint32_t da = tA + (uint32_t)(kb * 4 + k16) * 8;
                         const uint64_t db = dB0 + oB + (uint64_t)(kb * ((NT * 128) >> 4)) + k16 * 2;
                         asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                                     " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-                                     :: "r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"((uint32_t)((h | kb | k16) != 0)) : "memory");
+                                     " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+                                     :: "r"(tmem), "r"(da), "l"(db), "r"(idesc), "r"((uint32_t)((h | kb | k16) != 0)) : "memory");
                     }
                 }
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(&done16[h])) : "memory");
@@ -162,7 +168,7 @@ k_gemm_f16w(const __grid_constant__ GfParams p, const __grid_constant__ CUtensor
         if (elect_one()) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(&done_bar)) : "memory");
         __syncwarp();
     } else if (warp >= 4) {
-        // ---- converters: thread -> weight row r of its group's half-steps ----
+        // ---- converters: thread -> weight row r of its group's half-steps, the TMEM lane of its warp's quadrant ----
         const int r = (tid & 127), grp = (warp - 4) / GF_GROUP_WARPS;      // a quarter-warp = 8 consecutive rows: conflict-free swizzled accesses
         for (int h = grp; h < nhalf; h += GF_GROUPS) {
             const int g = h >> 1, half = h & 1;
@@ -185,11 +191,17 @@ k_gemm_f16w(const __grid_constant__ GfParams p, const __grid_constant__ CUtensor
                 }
             }
             if (h >= p.na) mbar_wait_spin(smem_u32(&done16[h - p.na]), 0, p.status, 28);      // the operand buffer is free again
-            unsigned char* dst = a16 + (size_t)(h % p.na) * GF_A16_BYTES + (size_t)r * 128;
+            __syncwarp();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t dst = tmem + ((uint32_t)((warp & 3) * 32) << 16) + NT + (uint32_t)(h % p.na) * GF_A_COLS;
             #pragma unroll
-            for (int q = 0; q < 16; ++q)             // k-block q / 8, eight k each
-                *reinterpret_cast<uint4*>(dst + (q >> 3) * 16384 + (((q & 7) ^ (r & 7)) << 4)) = o[q];
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // generic-proxy stores -> the MMA's async-proxy reads
+            for (int q = 0; q < 16; q += 4)          // 32 k: 16 columns
+                asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                             :: "r"(dst + (uint32_t)q * 4), "r"(o[q].x), "r"(o[q].y), "r"(o[q].z), "r"(o[q].w), "r"(o[q + 1].x), "r"(o[q + 1].y),
+                                "r"(o[q + 1].z), "r"(o[q + 1].w), "r"(o[q + 2].x), "r"(o[q + 2].y), "r"(o[q + 2].z), "r"(o[q + 2].w),
+                                "r"(o[q + 3].x), "r"(o[q + 3].y), "r"(o[q + 3].z), "r"(o[q + 3].w) : "memory");
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&a16_full[h]));
         }
@@ -222,7 +234,7 @@ k_gemm_f16w(const __grid_constant__ GfParams p, const __grid_constant__ CUtensor
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(NT < 32 ? 32 : NT));
+    if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(TMEM_COLS));
 }
 
 // One CTA per activation row: x (bf16 when !F32, else f32) -> fp16 row scaled by a power of two so that the
@@ -310,12 +322,10 @@ static int gf_launch(GfParams& p, const CUtensorMap& mx, const CUtensorMap& mw, 
     const size_t static_smem = (size_t)ac[1] - 1, room = (size_t)ac[0] - static_smem - 2048;
     const int nsup = p.K / 256, nhalf = p.K / 128;
     const size_t b_slot = 2 * (size_t)NT * 128;
-    // Shared memory: two fp16 operand buffers and three packed slots, the rest for the activation ring
-    // (measured: ring depths beyond these change nothing -- the kernel is bound by the conversion).
-    p.na = 2; p.sp = std::min(nsup, 3); p.sb = std::min(nhalf, 8);
-    auto need = [&] { return (size_t)p.na * GF_A16_BYTES + (size_t)p.sb * b_slot + (size_t)p.sp * GF_P_BYTES; };
+    // Shared memory: four packed slots, the rest for the activation ring.
+    p.na = GF_A_BUFS; p.sp = std::min(nsup, 4); p.sb = std::min(nhalf, 8);
+    auto need = [&] { return (size_t)p.sp * GF_P_BYTES + (size_t)p.sb * b_slot; };
     while (need() > room && p.sb > 2) --p.sb;
-    while (need() > room && p.sp > 2) --p.sp;
     if (need() > room) return B200_ENOTIMPL;
     p.na = std::min(p.na, nhalf);
     const size_t smem = need() + 1024;
