@@ -251,7 +251,7 @@ __device__ __forceinline__ int warp_sum_many(float (&v)[N], int lane) {
     return first;
 }
 template <int ET, int TM>
-__global__ void __launch_bounds__(GEMV_THREADS, 2)
+__global__ void __launch_bounds__(GEMV_THREADS, ET * TM > 64 ? 1 : 2)
 k_gemm_dense_rows(float* __restrict__ y, const __nv_bfloat16* __restrict__ W, const float* __restrict__ x, int M, int N, int K) {
     constexpr int OUT = ET * TM;
     __shared__ float part[GEMV_WARPS][OUT];
@@ -270,17 +270,18 @@ k_gemm_dense_rows(float* __restrict__ y, const __nv_bfloat16* __restrict__ W, co
             uint2 raw[ET];
             #pragma unroll
             for (int e = 0; e < ET; ++e) raw[e] = w0[min(e, ne) * k4 + 2 * i + h];
+            constexpr int XM = OUT > 64 ? TM : 4;     // activation rows loaded at a time: all of them where one CTA fills the SM
             #pragma unroll
-            for (int mh = 0; mh < TM; mh += 4) {
-                float4 xv[4];
+            for (int mh = 0; mh < TM; mh += XM) {
+                float4 xv[XM];
                 #pragma unroll
-                for (int m = 0; m < 4; ++m) xv[m] = x0[min(mh + m, nm) * k4 + 2 * i + h];
+                for (int m = 0; m < XM; ++m) xv[m] = x0[min(mh + m, nm) * k4 + 2 * i + h];
                 #pragma unroll
                 for (int e = 0; e < ET; ++e) {
                     const float wa = __uint_as_float(raw[e].x << 16), wb = __uint_as_float(raw[e].x & 0xffff0000u),
                                 wc = __uint_as_float(raw[e].y << 16), wd = __uint_as_float(raw[e].y & 0xffff0000u);
                     #pragma unroll
-                    for (int m = 0; m < 4; ++m) {
+                    for (int m = 0; m < XM; ++m) {
                         float& c = acc[e * TM + mh + m];
                         c = fmaf(wd, xv[m].w, fmaf(wc, xv[m].z, fmaf(wb, xv[m].y, fmaf(wa, xv[m].x, c))));
                     }
@@ -461,8 +462,13 @@ int dense_gemm(float* y, const void* W, const float* x, int M, int N, int K, int
     if (dtype != B200_F32 && dtype != B200_BF16) return B200_EINVAL;
     if (M > 8 && dtype == B200_BF16 && N <= 2048 && K >= 2048 && !(K & 7) && !((uintptr_t)W & 15) && !((uintptr_t)x & 15)) {
         // many rows against a small bf16 matrix (router logits of a prefill chunk): one launch, same bits per row
-        // 8 x 8 sums per thread once they fill the SMs twice over; below that smaller tiles and more CTAs
+        // 16 x 8 sums per thread, one CTA per SM, once there are four CTAs for every SM (the tail is then small): a tile brings
+        // 604 MB through L2 for 2048 rows against 144, an 8 x 8 one 906 MB, and that bounds it; a MoE layer of 2048 tokens
+        // 759 us with 8 x 8, 735 with these.  Below that 8 x 8, and while those are few too, smaller tiles and more CTAs.
         const __nv_bfloat16* w = static_cast<const __nv_bfloat16*>(W);
+        if ((long)((N + 15) / 16) * ((M + 7) / 8) >= 4L * sm_count())
+            k_gemm_dense_rows<16, 8><<<dim3((N + 15) / 16, (M + 7) / 8), GEMV_THREADS, 0, s>>>(y, w, x, M, N, K);
+        else
         if ((long)((N + 7) / 8) * ((M + 7) / 8) >= 4L * sm_count())
             k_gemm_dense_rows<8, 8><<<dim3((N + 7) / 8, (M + 7) / 8), GEMV_THREADS, 0, s>>>(y, w, x, M, N, K);
         else
