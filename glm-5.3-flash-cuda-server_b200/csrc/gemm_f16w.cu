@@ -25,7 +25,7 @@
 //   warp 2      TMEM allocation;  warps 12-15  at the end the epilogue: D[128 rows, NT tokens] * 2^e[token] / gs_w -> y
 // [4096 x 4096], 16 and 300 rows: 25.4 and 31.5 us with one group of eight converter warps, 22.5 and 28.4 with three groups
 // (about 2 us of it k_act_f16, eight elements a load instead of one), 19.5 and 25.7 with A in tensor memory; [12288 x 4096]
-// x 1024 rows 175, 166 and 150.
+// x 1024 rows 175, 166 and 150, and 107 with 256 tokens per tile.
 // Barriers are per step and used once (K <= 16384: 64 super-steps, 128 half-steps); every wait is bounded.
 // No cluster launch, no multicast.
 #include "b200_internal.h"
@@ -209,7 +209,7 @@ k_gemm_f16w(const __grid_constant__ GfParams p, const __grid_constant__ CUtensor
             // ---- epilogue ----
             const int te = tid - 384, q4 = warp & 3;
             pdl_wait();
-            if (te < NT) sx[te] = te < rows ? p.rowscale[m0 + te] / p.gs_w[0] : 0.f;
+            for (int c = te; c < NT; c += 128) sx[c] = c < rows ? p.rowscale[m0 + c] / p.gs_w[0] : 0.f;
             named_sync(1, 128);
             mbar_wait_spin(smem_u32(&done_bar), 0, p.status, 29);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -351,9 +351,12 @@ int gemm_f16w_dense(float* y, const b200_wref* W, const void* x, int x_kind, int
     if (((uintptr_t)W->packed & 15) || ((uintptr_t)W->scale & 15) || ((uintptr_t)x & 15) || ((uintptr_t)ws & 255)) return B200_ENOTIMPL;
     __half* xh = static_cast<__half*>(ws);
     float* rowscale = reinterpret_cast<float*>(static_cast<char*>(ws) + up256((size_t)M * K * 2));
-    // The conversion of a 128-row weight tile costs a CTA 9-12 us of the SFU pipe (cvt.e2m1x2 runs there), so it
-    // is shared by as many tokens as one accumulator holds; 64-token tiles were measured slower from 65 rows on.
-    const int NT = M <= 64 ? 64 : 128, n_jobs = (M + NT - 1) / NT, tiles_n = (N + 127) / 128;
+    // The conversion of a weight tile is shared by the tokens of one accumulator.  A wave of tiles of 256 tokens takes 1.43
+    // times one of 128 (K = 4096: 31.5 and 22 us), so 256 where that leaves at most 0.7 of the waves over the SMs:
+    // [12288 x 4096] 200 rows 58 -> 34 us (1 wave for 2), 512 rows 76.5 -> 70.6 (2 for 3), 1024 rows 150 -> 107 (3 for 6).
+    const int tiles_n = (N + 127) / 128;
+    auto waves = [&](int nt) { return ((long)tiles_n * ((M + nt - 1) / nt) + sm_count() - 1) / sm_count(); };
+    const int NT = M <= 64 ? 64 : 10 * waves(256) <= 7 * waves(128) ? 256 : 128, n_jobs = (M + NT - 1) / NT;
     GfParams p{};
     p.y = y; p.gs_w = W->gscale; p.rowscale = rowscale; p.status = device_status_ptr();
     if (!p.status) return B200_ENOTIMPL;
@@ -375,7 +378,8 @@ int gemm_f16w_dense(float* y, const b200_wref* W, const void* x, int x_kind, int
         if (e != cudaSuccess) return launch_failed("k_act_f16");
         if (int rc = check_launch("k_act_f16")) return rc;
     }
-    return NT == 64 ? gf_launch<64>(p, mx, mw, ms, tiles_n * n_jobs, s) : gf_launch<128>(p, mx, mw, ms, tiles_n * n_jobs, s);
+    const int grid = tiles_n * n_jobs;
+    return NT == 64 ? gf_launch<64>(p, mx, mw, ms, grid, s) : NT == 128 ? gf_launch<128>(p, mx, mw, ms, grid, s) : gf_launch<256>(p, mx, mw, ms, grid, s);
 }
 
 }  // namespace b200

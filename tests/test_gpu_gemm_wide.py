@@ -232,6 +232,18 @@ def test_gemm_bf16_exact_steps_over_converter_groups(M, N, K):
     test_gemm_bf16_exact_vs_oracle(M, N, K)
 
 
+@pytest.mark.parametrize('M,N,K', [(200, 12300, 256), (500, 6500, 768), (769, 9600, 1024)])
+def test_gemm_bf16_exact_tiles_of_256_tokens(M, N, K):
+    """Sizes that take 256 tokens per tile, the last tile ragged, and a row alone (64 per tile) equal to it bit for bit."""
+    test_gemm_bf16_exact_vs_oracle(M, N, K)
+    P = pkg()
+    W = P.Nvfp4Weight(*host_triple((N, K), 300 + N + K))
+    x = to_dev_bf16(bf16_rows(M, K, 9 + M))
+    y = P.gemm_bf16_exact(W, x)
+    for m in (0, 127, 128, M - 1):
+        assert torch.equal(P.gemm_bf16_exact(W, x[m:m + 1].contiguous())[0], y[m]), m
+
+
 def test_gemm_bf16_exact_rows_independent_and_repeatable():
     P = pkg()
     W = P.Nvfp4Weight(*host_triple((500, 1024), 77))

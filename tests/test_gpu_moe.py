@@ -361,6 +361,18 @@ def test_router_of_a_batch_equals_router_of_each_token_bitwise():
     assert torch.equal(l8, logits[:8])
 
 
+@pytest.mark.parametrize('E,M', [(144, 530), (100, 701), (129, 1000)])
+def test_router_of_a_long_chunk_equals_router_of_each_token_bitwise(E, M):
+    """The same with 16 experts x 8 tokens per CTA, ragged in both."""
+    P = pkg()
+    layer, d = build_layer(2048, 256, E, 8, seed=78, on_gpu=True)
+    x = torch.randn((M, 2048), device='cuda')
+    sel, wts, logits = P.moe_route(layer, x)
+    for m in (0, 7, 8, M // 2, M - 1):
+        s1, w1, l1 = P.moe_route(layer, x[m:m + 1].contiguous())
+        assert torch.equal(l1[0], logits[m]) and torch.equal(s1[0], sel[m]) and torch.equal(w1[0], wts[m]), m
+
+
 def test_byte_credit_reports_what_each_call_streams():
     """The profiler hook: host-known counts at the launch sites, device-side job counts after a flush
     (the contract of the reference's dprof_bytes / dprof_set_flush, include/dprof.h:83-103)."""
