@@ -63,3 +63,11 @@ def test_argument_checks_without_gpu():
     assert L.b200_moe_forward(16, C.byref(layer), 16, 16, 16, 16, 1, None) == 5   # n_expert > 512
     layer = pkg.MoeLayerC(pkg.WRef(16, None, None, None), 16, 16, None, 144, 8, 4100, 1536, 2.5, 10.0, 1)
     assert L.b200_moe_forward(16, C.byref(layer), 16, 16, 16, 16, 1, None) == 2
+
+
+def test_stable_weights_option_reaches_only_nvfp4_kernels():
+    """The option is a promise about NVFP4 weights.  A launch that takes plain matrices may not ask for it: it would read them
+    before its dependency wait without the caller having promised anything about them."""
+    src = os.path.join(ROOT, 'glm-5.3-flash-cuda-server_b200', 'csrc')
+    users = {f for f in os.listdir(src) if f.endswith('.cu') and 'stable_weights_option()' in open(os.path.join(src, f)).read()}
+    assert users == {'common.cu', 'gemv_tma.cu', 'gemv_umma.cu', 'gemm_mxf4.cu', 'gemm_f16w.cu', 'moe_stream.cu'}
