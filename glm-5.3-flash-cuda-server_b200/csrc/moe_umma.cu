@@ -3,8 +3,7 @@
 //
 // The expert tables of a layer live in device memory and the router picks experts on the device,
 // but a TMA tensor map has to be encoded on the host.  b200_moe_prepare therefore reads the
-// layer's tables once, encodes the six maps of every expert (gate, up, down: packed weights and
-// scales) and keeps them in device memory; at run time a small kernel turns (token, slot) pairs
+// layer's tables once, encodes the maps of every expert (moe_plan.cuh) and keeps them in device memory; at run time a small kernel turns (token, slot) pairs
 // into job records that point at the maps of the selected experts.
 //
 // Launches per layer up to 8 tokens: router logits, k_route (with the job records and the token rows' digits), gate and up
@@ -17,6 +16,7 @@
 // the slots in slot order.
 #include "b200_internal.h"
 #include "moe_plan.cuh"
+#include "moe_rows.h"
 #include "tma_pipe.cuh"
 #include <cstdio>
 #include <cstdlib>
@@ -40,9 +40,8 @@ static int group_min_tokens() {
 struct Prepared {
     const b200_nvfp4_mat* experts; const b200_nvfp4_mat* shared;     // key
     int E, H, I;
-    unsigned char* maps;          // device: [(E + 1) experts][3 matrices][w, s] x 128 bytes, shared expert last; then the same again
-                                  // with boxes 128 rows tall, for the wide GEMM (MU_GX_MAPS bytes further on)
-    int R_gu, R_d;
+    unsigned char* maps;          // device: MAPS_PER_EXPERT maps of every expert (moe_plan.cuh), shared expert last
+    MoeRows rows;
     int device;
 };
 static std::vector<Prepared> g_prepared;
@@ -61,18 +60,6 @@ static bool find_prepared(const b200_moe_layer* L, Prepared* out) {
             return true;
         }
     return false;
-}
-
-// Box height R for n_jobs jobs (one token's) of N rows in items of `boxes` * R: fewest waves of items over the SMs, each wave
-// costing its rows plus a fixed part (pipeline fill and drain) worth about 40 rows.
-static int pick_rows(int n_jobs, int N, int boxes) {
-    int best = 128; long best_cost = -1;
-    for (int R = 128; R >= 32; R -= 8) {
-        const long tasks = (long)n_jobs * ((N + boxes * R - 1) / (boxes * R)), waves = (tasks + sm_count() - 1) / sm_count();
-        const long cost = waves * (R + 40);
-        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = R; }
-    }
-    return best;
 }
 
 // y[m, h] = sum over the routed slots in slot order of wts[m, k] * part[row(m, k), h], plus the shared expert's
@@ -160,7 +147,7 @@ k_moe_group(const __grid_constant__ MoePlan q, UmJob* __restrict__ j1, UmJob* __
     }
     for (int e = threadIdx.x; e < G; e += blockDim.x) {
         const b200_nvfp4_mat* mats = e < q.E ? q.experts + (size_t)e * 3 : q.shared;
-        const unsigned char* mp = q.maps + (size_t)e * 6 * 128;
+        const unsigned char* mp = q.maps + ((size_t)e * MAPS_PER_EXPERT + MAP_CHUNK) * 128;
         for (int c = 0; c * 8 < cnt[e]; ++c) {
             const int idx = jstart[e] + c, rows = min(8, cnt[e] - 8 * c);
             const size_t pos0 = (size_t)off[e] + 8 * c;
@@ -232,7 +219,7 @@ int moe_umma_plan_args(const float* x, const b200_moe_layer* L, void* scratch, i
     q->part = reinterpret_cast<float*>(w); q->img1 = reinterpret_cast<unsigned char*>(w);
     q->experts = L->experts; q->shared = L->shared; q->maps = P->maps; q->x = x;
     q->topk = L->topk; q->ns = ns; q->E = L->n_expert; q->H = H; q->I = I;
-    *R_gu = P->R_gu; *R_d = P->R_d;
+    *R_gu = P->rows.stream_gu; *R_d = P->rows.stream_d;
     return B200_OK;
 }
 
@@ -269,9 +256,9 @@ static int moe_umma_grouped(const float* x, const b200_moe_layer* L, float* y, c
     k_moe_gather<<<(unsigned)((n4 + 255) / 256), 256, 0, s>>>(xg, x, posof, pairs, ns, H);
     if (int rc = check_launch("k_moe_gather")) return rc;
     if (int rc = umma_split_launch(s1, max_jobs, H, 0.f, s)) return rc;
-    if (int rc = umma_table_launch(j1, 2 * max_jobs, I, H, P->R_gu, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
+    if (int rc = umma_table_launch(j1, 2 * max_jobs, I, H, P->rows.chunk_gu, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
     if (int rc = umma_split_launch(s2, max_jobs, I, L->swiglu_limit, s)) return rc;
-    if (int rc = umma_table_launch(j2, max_jobs, H, I, P->R_d, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
+    if (int rc = umma_table_launch(j2, max_jobs, H, I, P->rows.chunk_d, s)) return rc == B200_ENOTIMPL ? B200_ELAUNCH : rc;
     return combine_launch(y, q.part, wts, posof, M, q.topk, ns, H, s);
 }
 
@@ -337,11 +324,11 @@ k_moe_group_gx(const __grid_constant__ MoePlan q, const int32_t* __restrict__ se
     for (int e = blockIdx.x + tid * gridDim.x; e < G; e += 1024 * gridDim.x) {
         const b200_nvfp4_mat* mats = e < q.E ? q.experts + (size_t)e * 3 : q.shared;
         const b200_nvfp4_mat g = mats[0], u = mats[1], d = mats[2];
-        const unsigned char* mp = q.maps + (size_t)(q.E + 1) * 6 * 128 + (size_t)e * 6 * 128;     // the 128-row boxes
+        const unsigned char* mp = q.maps + ((size_t)e * MAPS_PER_EXPERT + MAP_WIDE) * 128;
         for (int c = 0; c * NT < cnt[e]; ++c) {
             const int idx = jstart[e] + c, rows = min(NT, cnt[e] - NT * c), pos0 = off[e] + NT * c;
-            j1[idx] = GxJob{q.gbuf + (size_t)pos0 * q.I, g.gscale, u.gscale, gsx1 + pos0, mp, mp + 256, g.scale, u.scale, sf1 + idx * b1, pos0, rows, q.I, q.I};
-            j2[idx] = GxJob{q.part + (size_t)pos0 * q.H, d.gscale, nullptr, gsx2 + pos0, mp + 512, nullptr, d.scale, nullptr, sf2 + idx * b2, pos0, rows, q.H, q.H};
+            j1[idx] = GxJob{q.gbuf + (size_t)pos0 * q.I, g.gscale, u.gscale, gsx1 + pos0, mp, mp + 128, g.scale, u.scale, sf1 + idx * b1, pos0, rows, q.I, q.I};
+            j2[idx] = GxJob{q.part + (size_t)pos0 * q.H, d.gscale, nullptr, gsx2 + pos0, mp + 256, nullptr, d.scale, nullptr, sf2 + idx * b2, pos0, rows, q.H, q.H};
         }
     }
 }
@@ -441,20 +428,18 @@ extern "C" int b200_moe_prepare(const b200_moe_layer* L) {
     }
     Prepared P{};
     P.experts = L->experts; P.shared = L->shared; P.E = E; P.H = L->hidden; P.I = L->inter;
-    const int ns = L->topk + (L->shared ? 1 : 0);
-    P.R_gu = pick_rows(ns, L->inter, 1);
-    P.R_d = pick_rows(ns, L->hidden, 2);
-    std::vector<unsigned char> host((size_t)nexp * 12 * 128);
+    P.rows = moe_rows(L->topk, L->shared != nullptr, E, L->hidden, L->inter, sm_count());
+    std::vector<unsigned char> host((size_t)nexp * MAPS_PER_EXPERT * 128);
     for (int e = 0; e < nexp; ++e) {
         const b200_nvfp4_mat* m = &mats[(size_t)e * 3];
-        unsigned char* o = host.data() + (size_t)e * 6 * 128;
-        if (umma_encode_maps(o, o + 128, m[0].packed, m[0].scale, L->inter, L->hidden, P.R_gu) ||
-            umma_encode_maps(o + 256, o + 384, m[1].packed, m[1].scale, L->inter, L->hidden, P.R_gu) ||
-            umma_encode_maps(o + 512, o + 640, m[2].packed, m[2].scale, L->hidden, L->inter, P.R_d)) return B200_ENOTIMPL;
-        o += (size_t)nexp * 6 * 128;                     // the wide GEMM's boxes: always 128 rows
-        if (umma_encode_maps(o, o + 128, m[0].packed, m[0].scale, L->inter, L->hidden, 128) ||
-            umma_encode_maps(o + 256, o + 384, m[1].packed, m[1].scale, L->inter, L->hidden, 128) ||
-            umma_encode_maps(o + 512, o + 640, m[2].packed, m[2].scale, L->hidden, L->inter, 128)) return B200_ENOTIMPL;
+        unsigned char* o = host.data() + (size_t)e * MAPS_PER_EXPERT * 128;
+        for (int q = 0; q < 3; ++q) {
+            const int N = q < 2 ? L->inter : L->hidden, K = q < 2 ? L->hidden : L->inter;
+            unsigned char* chunk = o + (MAP_CHUNK + 2 * q) * 128;
+            if (umma_encode_maps(chunk, chunk + 128, m[q].packed, m[q].scale, N, K, q < 2 ? P.rows.chunk_gu : P.rows.chunk_d) ||
+                !tmap_u8_2d(o + (MAP_STREAM + q) * 128, m[q].packed, (size_t)N, (size_t)K / 2, 128, q < 2 ? P.rows.stream_gu : P.rows.stream_d, true, false) ||
+                !tmap_u8_2d(o + (MAP_WIDE + q) * 128, m[q].packed, (size_t)N, (size_t)K / 2, 128, 128, true, false)) return B200_ENOTIMPL;
+        }
     }
     if (cudaGetDevice(&P.device) != cudaSuccess) return launch_failed("moe_prepare: cudaGetDevice");
     if (cudaMalloc(&P.maps, host.size()) != cudaSuccess) return launch_failed("moe_prepare: cudaMalloc");
