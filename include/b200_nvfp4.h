@@ -104,9 +104,11 @@ int b200_nvfp4_selftest_bounded_wait(b200_stream stream);
 /* Process-wide options.  B200_OPT_STABLE_WEIGHTS = 1 declares that no kernel running on a
  * stream writes NVFP4 weight buffers that a later call on that stream reads (true for an
  * inference engine, whose weights are loaded once).  The pipelined kernels, which are launched
- * with programmatic stream serialisation, may then start copying weights while the previous
- * kernel of the stream is still finishing; activations, scales and outputs are still only
- * touched after the previous kernel has completed.  Default 0 (also settable with the
+ * with programmatic stream serialisation, may then start reading weights while the previous
+ * kernel of the stream is still finishing: the packed codes and their block scales, which are
+ * one matrix.  Everything else -- activations, global scales, plain bf16 or f32 matrices (a
+ * router's too), biases, selections, gates and outputs -- is only touched after the previous
+ * kernel has completed.  Default 0 (also settable with the
  * environment variable B200_STABLE_WEIGHTS=1).  No counterpart in the reference. */
 /* B200_OPT_PREFILL_FP4 (default 1; environment B200_PREFILL_FP4=0 turns it off): calls that carry
  * scratch and 16 or more activation rows -- b200_nvfp4_gemm_ws with M >= 16, the MoE block with 16
