@@ -18,7 +18,7 @@
 // products and sums inside the MMA are exact / fp32.
 //
 // Per CTA (one per SM): T consecutive tiles of R rows of one job (R <= 128 a multiple of 8; T = 1
-// for a plain gemv, up to 8 for the MoE job-table launches), K walked in steps of 256.
+// but for calls of more than two tiles of 128 rows per SM, which take up to 8), K walked in steps of 256.
 //   warp 0      TMA producer.  First the CTA's scale rows, as slabs [R rows x 128 B] (128B-swizzled,
 //               so 32 lanes reading one 16-byte column of 32 consecutive rows hit different banks);
 //               then per step one box [128 B x R rows] of packed weights (SWIZZLE_128B, the K-major

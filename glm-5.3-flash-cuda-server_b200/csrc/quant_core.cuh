@@ -5,7 +5,7 @@
 // every step is one IEEE fp32 operation in the reference's order (__fdiv_rn / __fmul_rn, so that
 // the compiler cannot fuse or reorder them), and code selection is numpy's searchsorted(mid, v) =
 // "number of mid-points strictly below v", so a value exactly on a mid-point takes the LOWER code
-// (the hardware converters round such ties to even, which is why they are not used here).
+// (the hardware converter rounds such ties to even: quantize_codes says where it is used all the same).
 #pragma once
 #include "nvfp4_decode.cuh"
 

@@ -1,5 +1,7 @@
-"""The quantisers where their fast paths hand over: elements within rounding distance of a mid-point, steps outside the range
-of the fast reciprocal, outputs too unaligned for the maximum's scratch words, and one-row tensors.  Bit for bit the oracle."""
+"""The quantisers where their fast paths hand over (f32 rows: two conversions per element, and comparisons for a group in which they
+differ): elements within rounding distance of a mid-point, steps outside the range of the fast reciprocal; bf16 tensors, which are
+compared throughout: elements at their thresholds, outputs too unaligned for the maximum's scratch words, one-row tensors.  Bit for
+bit the oracle."""
 import numpy as np
 import pytest
 import torch
@@ -65,8 +67,8 @@ def test_quantize_with_unaligned_outputs(N, K, off):
 @pytest.mark.parametrize('exp', [0, 20, -20])
 @pytest.mark.parametrize('off', list(range(-12, 13, 2)) + [7, 9])
 def test_bf16_elements_next_to_mid_points(off, exp):
-    """Steps a few ulps off a short mantissa, so that mid-points times the step lie that close to bf16 numbers: where the one
-    conversion per element hands over to the comparisons, and just outside."""
+    """Steps a few ulps off a short mantissa, so that mid-points times the step lie that close to bf16 numbers: there the
+    thresholds rounded down to bf16 decide the packed comparisons."""
     P, O = pkg(), oracle()
     rng, N, K = np.random.default_rng(off + 100), 16, 512
     gs = np.array([(np.float32(2.0 ** -exp).view(np.int32) + off)], np.int32).view(np.float32)
