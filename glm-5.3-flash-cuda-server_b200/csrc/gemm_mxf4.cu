@@ -11,10 +11,11 @@
 //
 // Persistent: one CTA per SM walks work items (TA tiles of R <= 128 weight rows) x (a job's NT tokens), K in steps of
 // 256.  The accumulators D[128 weight rows (lanes), NT tokens (columns)] of the TA tiles stay in TMEM for the whole K.
-// What bounds it is the SM's intake from L2, about 64 B per clock: a step of a 128 x NT tile brings 16 KB of weights and
-// NT x 128 B of activations for NT/2 clocks of MMA.  Hence TA = 2: two weight tiles against one activation tile
-// (for a MoE expert its gate and its up tile, so that the SwiGLU is applied where both sums lie and one value instead
-// of two is written).
+// A step of a 128 x NT tile brings 16 KB of weights and NT x 128 B of activations for NT/2 clocks of MMA.  Hence TA = 2: two
+// weight tiles against one activation tile (for a MoE expert its gate and its up tile, so that the SwiGLU is applied where
+// both sums lie and one value instead of two is written).  Bound by HBM for the experts of 512 tokens (5.1 TB/s read).  A dense
+// call of one item per CTA ([12288 x 4096] x 512) is at no unit's limit: over a CTA's life its SM takes in 29 B per clock from
+// L2 and the tensor pipe is active a third of the time.
 //   warp 0      TMA: per step TA 128B-swizzled boxes of packed weights [128 B x R]
 //   warp 3      TMA: per step one box of packed activations [128 B x NT] and their scale bytes (one bulk copy: the
 //               quantiser writes them in the order tcgen05.cp wants)
@@ -476,6 +477,8 @@ size_t gemm_mxf4_ws_bytes(int M, int K) {
     return up256(rows * (size_t)(K / 2)) + up256(dense_sf_rows(M) * (size_t)(K / 16)) + up256(rows * 4);
 }
 
+// scale_box: this kernel has no scale slabs and could do without it, but calls reach it by their row count too
+// (b200_nvfp4_gemm_ws), and at the K that it leaves out (4352, say) they give exact products at every M.
 bool gemm_mxf4_shape_ok(int K) {
     int b, z;
     return !(K & 255) && K >= 256 && K <= 16384 && scale_box(K, &b, &z) && tmap_available();
