@@ -536,7 +536,7 @@ static int gx_launch(const GxParams& p, const GxMaps& maps, int grid, size_t sme
     return p.nblk == 1 ? gx_launch_n<TABLE, TA, DUAL, 1>(p, maps, grid, smem, s) : gx_launch_n<TABLE, TA, DUAL, 2>(p, maps, grid, smem, s);
 }
 
-// Shape of a dense call's items: (R, TA, NT) with the least estimated time.  An SM takes in about 115 B per ns and its
+// Shape of a dense call's items: (R, TA, NT) with the least estimated time.  The model: an SM takes in 115 B per ns and its
 // tensor pipe needs NT/2 clocks per 128 x NT x 64; a wave of items costs its steps at the slower of the two, plus its
 // epilogue where no second accumulator set hides it (5 ns per column and tile).  So few tokens get weight tiles just
 // low enough to give every SM one, and many get two 128-row tiles against a chunk of tokens that fills whole waves:
